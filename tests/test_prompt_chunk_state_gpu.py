@@ -1,0 +1,49 @@
+"""What a chunked prompt leaves behind: all of the state and outputs that the token-by-token walk leaves."""
+import pytest
+import torch
+
+from tests.helpers import assert_close_at_scale
+from tilefoundry_b200.authored import qwen3_5_35b_a3b as q35
+from tilefoundry_b200.authored.weights import random_weights
+from tilefoundry_b200.runtime import DictResource
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def qwen35():
+    """``session(n_prompt) -> (session, prompt)`` over one set of weights whose rounding flips no expert that counts."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from tilefoundry_b200 import lib
+    from tilefoundry_b200.engine.qwen3_5 import Qwen35Session
+    lib.load()
+    cfg = q35.QWEN3_5_TINY
+    w = random_weights(q35.build(cfg), seed=9, std=0.05, overrides=q35.weight_overrides)
+    for name, t in w.items():
+        leaf = name.rsplit(".", 1)[-1]
+        t *= 0.02 if leaf in ("w_o", "w_out", "w_down", "w_shared_down") else 3.0 if leaf == "w_router" else 1.0
+    res = DictResource({k: v.to("cuda:0") for k, v in w.items()})
+
+    def session(n_prompt):
+        sess = Qwen35Session(cfg, res, max_ctx=128, device="cuda:0", keep_logits=True)
+        return sess, torch.randint(0, cfg.vocab_size, (n_prompt,), generator=torch.Generator().manual_seed(n_prompt))
+    return session
+
+
+# chunks of 2 and 3 reach back into the window before them; odd and even lengths and starts swap the two windows' buffers
+@pytest.mark.parametrize("pieces", [(2,), (3,), (4,), (17,), (40,), (2, 2), (2, 3), (3, 2), (5, 4), (16, 21)])
+def test_chunks_leave_both_convolution_windows(qwen35, pieces):
+    (walk, prompt), (pre, _) = qwen35(sum(pieces) + 1), qwen35(sum(pieces) + 1)
+    walk.reset(prompt), pre.reset(prompt)
+    for _ in range(sum(pieces)):
+        walk.step()
+    for n in pieces:
+        pre.prefill(n)
+    pre._prefill.check_status()
+    assert int(pre.pos) == int(walk.pos) == sum(pieces)
+    assert len(pre.state_tensors()) == len(walk.state_tensors()) > 0
+    for i, (got, want) in enumerate(zip(pre.state_tensors(), walk.state_tensors())):
+        assert got.shape == want.shape
+        for part, (a, b) in enumerate(zip(got, want)):      # a window, or a head's state, at its own scale
+            assert_close_at_scale(a, b, f"state tensor {i} part {part}")

@@ -184,20 +184,25 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const GdnChunkParams p) 
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int q = 0; q < 4; ++q) state[size_t(16 * i + 4 * part + q) * 128] = s[i][q];
-    // the window the next token reads: the last three entries, in the buffer of its position's parity (every reader of the
-    // old window was in the kernel before this one)
+    // Both windows, as the walk leaves them: the one the next token reads (the last three entries, in the buffer of its
+    // position's parity) and the one before it (a session's state is both buffers).  Every reader of the old window was in the
+    // kernel before this one; a thread has its channel's old entries in registers before it writes either buffer.
     const float* win = p.conv_state + size_t(pos0 & 1) * p.conv_state_stride;
-    float* out = p.conv_state + size_t((pos0 + p.m) & 1) * p.conv_state_stride;
+    float* next = p.conv_state + size_t((pos0 + p.m) & 1) * p.conv_state_stride;
+    float* last = p.conv_state + size_t((pos0 + p.m + 1) & 1) * p.conv_state_stride;
     const int conv = 2 * key + val, ctas = gridDim.x * gridDim.y;
     for (int c = (blockIdx.y * gridDim.x + blockIdx.x) * 128 + tid; c < conv; c += ctas * 128) {
-        float e[3];
+        float e[4];                                       // entries m - 4 .. m - 1; a negative one is of the old window
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const int at = p.m - 3 + j;
+        for (int j = 0; j < 4; ++j) {
+            const int at = p.m - 4 + j;                   // (m >= 2: not below -2)
             e[j] = at >= 0 ? bf16_bits_to_f32(p.proj[size_t(at) * p.proj_width + c]) : win[size_t(c) * 3 + at + 3];
         }
 #pragma unroll
-        for (int j = 0; j < 3; ++j) out[size_t(c) * 3 + j] = e[j];
+        for (int j = 0; j < 3; ++j) {
+            next[size_t(c) * 3 + j] = e[j + 1];
+            last[size_t(c) * 3 + j] = e[j];
+        }
     }
 }
 
