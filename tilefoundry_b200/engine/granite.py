@@ -198,7 +198,8 @@ class GraniteSession(DecodeSession):
         return total
 
     def state_bytes(self) -> int:
-        c = self.cfg
+        """Recurrent state read and written per token."""
+        c, n_m = self.cfg, sum(l["kind"] == "linear_attention" for l in self.layers)
         return n_m * 2 * c.mamba_n_heads * c.mamba_d_head * c.mamba_d_state * 4
 
     def kv_bytes_per_position(self) -> int:
