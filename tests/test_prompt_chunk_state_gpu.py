@@ -47,3 +47,24 @@ def test_chunks_leave_both_convolution_windows(qwen35, pieces):
         assert got.shape == want.shape
         for part, (a, b) in enumerate(zip(got, want)):      # a window, or a head's state, at its own scale
             assert_close_at_scale(a, b, f"state tensor {i} part {part}")
+
+
+@pytest.mark.parametrize("use_graph", [False, True])
+def test_steps_inside_a_prompt_leave_their_logits_and_picks(qwen35, use_graph):
+    """``run`` takes every position as a step, also at the start of a sequence: a caller who scores a prompt piece by piece
+    reads each piece's last logits and pick, and nothing waits for the device."""
+    (walk, prompt), (sess, _) = qwen35(10), qwen35(10)
+    walk.reset(prompt)
+    sess.generate(prompt.flip(0), 1)                     # another request's logits and pick lie there
+    sess.reset(prompt)
+    for steps in (5, 3, 2):                              # inside the prompt, and its end
+        for _ in range(steps):
+            walk.step()
+        torch.cuda.set_sync_debug_mode("error")          # (a device read inside run raises)
+        try:
+            sess.run(steps, use_graph)
+        finally:
+            torch.cuda.set_sync_debug_mode("default")
+        assert torch.equal(sess.logits, walk.logits) and int(sess.picked) == int(walk.picked) and int(sess.pos) == int(walk.pos)
+    for got, want in zip(sess.state_tensors(), walk.state_tensors()):
+        assert torch.equal(got, want)

@@ -210,7 +210,6 @@ class Qwen35Session(DecodeSession):
         for layer in self._recurrent():               # recurrent state starts at zero for a new sequence
             layer["conv_state"].zero_()
             layer["state"].zero_()
-        self._fresh = True
 
     def state_tensors(self) -> list:
         return [l[n] for l in self._recurrent() for n in ("conv_state", "state")]
@@ -238,7 +237,6 @@ class Qwen35Session(DecodeSession):
         return 2 * c.n_kv_heads * c.head_dim * 4 * (len(self.layers) - len(self._recurrent()))
 
     def step(self) -> None:
-        self._fresh = False
         so = lib.load()
         if self.world == 1:
             lib.check(so.tfb_qwen35_decode_step(C.byref(self.args), lib.stream()), "tfb_qwen35_decode_step")
@@ -256,13 +254,11 @@ class Qwen35Session(DecodeSession):
         chunk) instead of one decode step each, and advance the position.  Nothing is picked.  One GPU only."""
         if not self._chunked():
             raise ValueError("chunked prompt processing is not built for this session")
-        self._fresh = False
         self._chunks().run(n_tokens, first)
 
     def _take_prompt(self, max_new: int, use_graph: bool, mid) -> int:
-        if not (max_new > 0 and self.n_prompt >= 3 and self._fresh and self.trace is None and self._chunked()):
+        if not (max_new > 0 and self.n_prompt >= 3 and self.trace is None and self._chunked()):
             return super()._take_prompt(max_new, use_graph, mid)
-        self._fresh = False
         return self._prompt_in_chunks(self._chunks(), max_new, mid)
 
     def _chunks(self):
@@ -277,34 +273,9 @@ class Qwen35Session(DecodeSession):
         lib.check(lib.load().tfb_qwen35_step_part(C.byref(tail), 3, 0, lib.stream()), "tfb_qwen35_step_part")
 
     _prefill = None
-    _fresh = False                                   # nothing has run since ``reset``
 
     def _chunked(self) -> bool:
         return self.world == 1 and bool(lib.load().tfb_qwen35_prefill_supported(C.byref(self.args)))
-
-    def restore(self, snap: dict) -> None:
-        super().restore(snap)
-        self._fresh = False
-
-    def capture(self) -> None:
-        fresh = self._fresh
-        super().capture()                            # (its warm-up steps are rolled back)
-        self._fresh = fresh
-
-    def run(self, steps: int, use_graph: bool = True) -> None:
-        """As DecodeSession.run; at the start of a sequence the prompt positions among the *steps* go through in chunks
-        (every weight read once per chunk: a 64-token prompt takes 10 times less than 64 steps).  A chunk costs about as
-        much as one or two steps, and a session that records a trace takes every step by itself."""
-        if self._fresh and steps >= 3 and self.trace is None and self._chunked():
-            self._fresh = False
-            first = int(self.pos.item())
-            known = min(steps, self.n_prompt - first)
-            if known >= 3:
-                last = self._chunks().run(known, first, pick=known == self.n_prompt - first)
-                if last is not None:                  # (the whole prompt: its last token's successor is picked, as in generate)
-                    self._pick_from(last)
-                steps -= known
-        super().run(steps, use_graph)
 
     def check_prompt(self) -> None:
         if self._prefill is not None:
