@@ -3,6 +3,8 @@ import pytest
 import torch
 
 from tests.helpers import assert_close_at_scale
+from tilefoundry_b200.authored import minicpm3_4b as mc
+from tilefoundry_b200.authored import qwen3_1_7b as q
 from tilefoundry_b200.authored import qwen3_5_35b_a3b as q35
 from tilefoundry_b200.authored.weights import random_weights
 from tilefoundry_b200.runtime import DictResource
@@ -68,3 +70,37 @@ def test_steps_inside_a_prompt_leave_their_logits_and_picks(qwen35, use_graph):
         assert torch.equal(sess.logits, walk.logits) and int(sess.picked) == int(walk.picked) and int(sess.pos) == int(walk.pos)
     for got, want in zip(sess.state_tensors(), walk.state_tensors()):
         assert torch.equal(got, want)
+
+
+def _chunked_session(model, qwen35):
+    if model == "qwen3.5":
+        return qwen35(8)
+    from tilefoundry_b200.engine.minicpm3 import MiniCPM3Session
+    from tilefoundry_b200.engine.qwen3 import Qwen3Session
+    mod, cfg, cls = (q, q.QWEN3_SMALL, Qwen3Session) if model == "qwen3" else (mc, mc.MINICPM3_TINY, MiniCPM3Session)
+    w = mod.tie_head(random_weights(mod.build(cfg), seed=7, std=0.02))
+    sess = cls(cfg, DictResource({k: v.to("cuda:0") for k, v in w.items()}), max_ctx=64, device="cuda:0")
+    return sess, torch.randint(0, cfg.vocab_size, (8,), generator=torch.Generator().manual_seed(8))
+
+
+@pytest.mark.parametrize("model", ["qwen3", "minicpm3", "qwen3.5"])
+def test_a_given_up_wait_of_a_chunk_is_told_once(model, qwen35):
+    """The status word as a kernel that gave up leaves it (set from the host): the next call that waits for the stream raises."""
+    sess, prompt = _chunked_session(model, qwen35)
+    token_in, token_out = (torch.zeros(1, dtype=torch.int64).pin_memory() for _ in range(2))
+    calls = {"step_host": lambda: sess.step_host(6, token_in, token_out), "generate_host": lambda: sess.generate_host(6, 1, token_in),
+             "check_prompt": sess.check_prompt}
+    for call in calls.values():
+        sess.reset(prompt)
+        sess.prefill(6)
+        sess._prefill.status.fill_(2)
+        with pytest.raises(RuntimeError, match="bounded wait"):
+            call()
+        call()                                           # told once
+    assert not sess.prompt_unchecked
+    sess.reset(prompt)
+    sess.prefill(6)
+    sess._prefill.status.fill_(2)
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        sess.generate(prompt, 2, prefill=True) if model != "qwen3.5" else sess.generate(prompt, 2)
+    assert len((sess.generate(prompt, 2, prefill=True) if model != "qwen3.5" else sess.generate(prompt, 2)).tokens) == 2

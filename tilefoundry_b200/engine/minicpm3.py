@@ -176,7 +176,7 @@ class MiniCPM3Session(DecodeSession):
         from .minicpm3_prefill import MiniCPM3Prefill
         if self.cache != "latent":
             raise ValueError("chunked prompt processing is built for the latent cache")
-        if getattr(self, "_prefill", None) is None:
+        if self._prefill is None:
             self._prefill = MiniCPM3Prefill(self)
         return self._prefill
 
@@ -204,6 +204,6 @@ class MiniCPM3Session(DecodeSession):
         self.run(max_new - picked, use_graph)
         end.record()
         torch.cuda.synchronize()
-        self._prefill.check_status()
+        self.check_prompt()
         out = self.tokens[self.n_prompt: self.generated_end(self.n_prompt + max_new)].tolist()
         return Generated(out, mid.elapsed_time(end) / 1e3, start.elapsed_time(mid) / 1e3, self.n_prompt)

@@ -191,7 +191,7 @@ class Qwen3Session(DecodeSession):
 
     def _chunks(self):
         from .qwen3_prefill import Qwen3Prefill
-        if getattr(self, "_prefill", None) is None:
+        if self._prefill is None:
             self._prefill = Qwen3Prefill(self)
         return self._prefill
 
@@ -225,6 +225,6 @@ class Qwen3Session(DecodeSession):
         self.run(max_new - picked, use_graph)
         end.record()
         torch.cuda.synchronize()
-        self._prefill.check_status()
+        self.check_prompt()
         out = self.tokens[self.n_prompt: self.generated_end(self.n_prompt + max_new)].tolist()
         return Generated(out, mid.elapsed_time(end) / 1e3, start.elapsed_time(mid) / 1e3, self.n_prompt)

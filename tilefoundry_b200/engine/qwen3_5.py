@@ -272,11 +272,5 @@ class Qwen35Session(DecodeSession):
         tail.hidden_buf = hidden
         lib.check(lib.load().tfb_qwen35_step_part(C.byref(tail), 3, 0, lib.stream()), "tfb_qwen35_step_part")
 
-    _prefill = None
-
     def _chunked(self) -> bool:
         return self.world == 1 and bool(lib.load().tfb_qwen35_prefill_supported(C.byref(self.args)))
-
-    def check_prompt(self) -> None:
-        if self._prefill is not None:
-            self._prefill.check_status()

@@ -61,6 +61,7 @@ class Qwen3Prefill:
         first = int(sess.pos.item()) if first is None else first
         if n_tokens < 0 or first + n_tokens > sess.max_ctx:
             raise ValueError(f"{first}+{n_tokens} tokens exceed capacity {sess.max_ctx}")
+        sess.prompt_unchecked = True
         done = 0
         while n_tokens - done >= 2:
             m = min(self.chunk, n_tokens - done)
@@ -82,4 +83,5 @@ class Qwen3Prefill:
     def check_status(self) -> None:
         code = int(self.status.item())
         if code:
+            self.status.zero_()                          # told once
             raise RuntimeError(f"a bounded wait of a prompt chunk's kernels gave up (status {code})")

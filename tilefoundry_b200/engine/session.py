@@ -30,6 +30,8 @@ class DecodeSession:
     prompt_word = None
     eos_ids = None
     stop_at = None
+    _prefill = None                                   # the chunk processor, once a prompt went through it
+    prompt_unchecked = False                          # a prompt went through in chunks whose status nobody has read
 
     def step(self) -> None:
         raise NotImplementedError
@@ -138,6 +140,8 @@ class DecodeSession:
         lib.check(lib.load().tfb_graph_step_host(int(self.graph.raw_cuda_graph_exec()), base + 8 * pos, token_in.data_ptr(),
                                                  base + 8 * (pos + 1), token_out.data_ptr(), lib.stream()),
                   "tfb_graph_step_host")
+        if self.prompt_unchecked:
+            self.check_prompt()
 
     def generate_host(self, pos: int, steps: int, token_io: torch.Tensor) -> list:
         """*steps* iterations of ``step_host`` from position *pos* in one C call: ``token_io`` (pinned int64[1]) holds the
@@ -152,6 +156,8 @@ class DecodeSession:
         lib.check(lib.load().tfb_graph_generate_host(int(self.graph.raw_cuda_graph_exec()), self.tokens.data_ptr(), pos, steps,
                                                      token_io.data_ptr(), out.data_ptr(), lib.stream()),
                   "tfb_graph_generate_host")
+        if self.prompt_unchecked:
+            self.check_prompt()
         return out[:steps].tolist()
 
     def run(self, steps: int, use_graph: bool = True) -> None:
@@ -161,7 +167,13 @@ class DecodeSession:
             self.graph.replay() if use_graph else self.step()
 
     def check_prompt(self) -> None:
-        """Raise if a prompt taken in chunks left void results (called once the stream has finished)."""
+        """Raise if a prompt taken in chunks left void results: a bounded wait of its kernels gave up.  Waits for the stream.
+        ``generate``, ``step_host`` and ``generate_host`` call it, the latter two once after a ``prefill``; a caller who
+        only enqueues (``prefill``, ``run``) calls it when the stream has finished.  An error is raised once: the next
+        prompt starts clean."""
+        self.prompt_unchecked = False
+        if self._prefill is not None:
+            self._prefill.check_status()
 
     def generate(self, prompt_ids, max_new: int, use_graph: bool = True, eos=None) -> Generated:
         """Walk the prompt, then continue greedily for *max_new* tokens; one sync at each end.  *eos*: token ids
@@ -180,7 +192,8 @@ class DecodeSession:
         self.run(max_new - picked, use_graph)      # step at position p writes token p+1
         end.record()
         torch.cuda.synchronize()
-        self.check_prompt()
+        if self.prompt_unchecked:
+            self.check_prompt()
         out = self.tokens[n_prompt: self.generated_end(n_prompt + max_new)].tolist()
         return Generated(out, mid.elapsed_time(end) / 1e3, start.elapsed_time(mid) / 1e3, n_prompt)
 
