@@ -675,10 +675,10 @@ def side_config(key, dev, K, W, with_cpu):
     out = {"workload": work.describe, "dtype": work.dtype, "unit": "tok/s", **m, "roofline": roofline_of(work, sess, whole)}
     if hasattr(sess, "prefill"):
         # prompt processing, outside the metric: the 64-token prompt walked one decode step per token against the
-        # same prompt in chunks of 32 tokens (tensor-core projections)
+        # same prompt in one chunk
         try:
             prompt = prompt_ids(work.cfg, 0)
-            walk = sess.generate(prompt, 4)
+            walk = sess.generate(prompt, 4, prefill=False)
             sess.generate(prompt, 4, prefill=True)                                  # warm-up: buffers, tensor maps
             chunked = sess.generate(prompt, 4, prefill=True)
             out["prompt"] = {"tokens": PROMPT_TOKENS, "walk_ms": walk.prompt_seconds * 1e3,
@@ -773,7 +773,7 @@ def run_ours(args):
         # prompt in chunks of 32 tokens on the tensor-core projections (Qwen3 only)
         prompt_info = batch32 = None
         if world == 1 and hasattr(sess, "prefill") and not args.no_sides:
-            walk = sess.generate(prompt, 4)
+            walk = sess.generate(prompt, 4, prefill=False)
             sess.generate(prompt, 4, prefill=True)                                  # warm-up: buffers, tensor maps
             chunked = sess.generate(prompt, 4, prefill=True)
             prompt_info = {"tokens": PROMPT_TOKENS, "walk_ms": walk.prompt_seconds * 1e3,

@@ -102,5 +102,16 @@ def test_a_given_up_wait_of_a_chunk_is_told_once(model, qwen35):
     sess.prefill(6)
     sess._prefill.status.fill_(2)
     with pytest.raises(RuntimeError, match="bounded wait"):
-        sess.generate(prompt, 2, prefill=True) if model != "qwen3.5" else sess.generate(prompt, 2)
-    assert len((sess.generate(prompt, 2, prefill=True) if model != "qwen3.5" else sess.generate(prompt, 2)).tokens) == 2
+        sess.generate(prompt, 2, prefill=True)
+    assert len(sess.generate(prompt, 2, prefill=True).tokens) == 2
+
+
+@pytest.mark.parametrize("model", ["qwen3", "minicpm3", "qwen3.5"])
+def test_generate_is_asked_for_chunks_or_a_walk(model, qwen35):
+    """``prefill`` of ``generate`` on every session that has chunks; without it each keeps its own default."""
+    sess, prompt = _chunked_session(model, qwen35)
+    walked = sess.generate(prompt, 3, prefill=False)
+    assert sess._prefill is None and walked.prompt_steps == 8
+    assert sess.generate(prompt, 3, True, None if model == "qwen3.5" else False).prompt_steps == 8      # (the fourth argument as before)
+    chunked = sess.generate(prompt, 3, prefill=True)
+    assert sess._prefill is not None and len(chunked.tokens) == len(walked.tokens) == 3 and int(sess.pos) == 10

@@ -210,21 +210,4 @@ class Qwen3Session(DecodeSession):
 
     def generate(self, prompt_ids, max_new: int, use_graph: bool = True, prefill: bool = False, eos=None):
         """As DecodeSession.generate; with ``prefill`` the prompt is processed in chunks."""
-        if not prefill:
-            return super().generate(prompt_ids, max_new, use_graph, eos)
-        if eos is not None:
-            self.set_eos(eos)
-        self.reset(prompt_ids)
-        if self.n_prompt + max_new > self.max_ctx + 1:
-            raise ValueError(f"{self.n_prompt}+{max_new} tokens exceed capacity {self.max_ctx}")
-        if use_graph and self.graph is None:
-            self.capture()
-        start, mid, end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
-        start.record()
-        picked = self._prompt_in_chunks(self._chunks(), max_new, mid)
-        self.run(max_new - picked, use_graph)
-        end.record()
-        torch.cuda.synchronize()
-        self.check_prompt()
-        out = self.tokens[self.n_prompt: self.generated_end(self.n_prompt + max_new)].tolist()
-        return Generated(out, mid.elapsed_time(end) / 1e3, start.elapsed_time(mid) / 1e3, self.n_prompt)
+        return self._generate(prompt_ids, max_new, use_graph, eos, self._chunk_prompt if prefill else self._walk_prompt)

@@ -256,10 +256,14 @@ class Qwen35Session(DecodeSession):
             raise ValueError("chunked prompt processing is not built for this session")
         self._chunks().run(n_tokens, first)
 
+    def generate(self, prompt_ids, max_new: int, use_graph: bool = True, eos=None, *, prefill: bool = True):
+        """As DecodeSession.generate.  The prompt goes through in chunks where the session has them and a token is picked
+        after it (``prefill=False``: token by token)."""
+        return self._generate(prompt_ids, max_new, use_graph, eos, self._take_prompt if prefill else self._walk_prompt)
+
     def _take_prompt(self, max_new: int, use_graph: bool, mid) -> int:
-        if not (max_new > 0 and self.n_prompt >= 3 and self.trace is None and self._chunked()):
-            return super()._take_prompt(max_new, use_graph, mid)
-        return self._prompt_in_chunks(self._chunks(), max_new, mid)
+        chunks = max_new > 0 and self.n_prompt >= 3 and self.trace is None and self._chunked()
+        return (self._chunk_prompt if chunks else self._walk_prompt)(max_new, use_graph, mid)
 
     def _chunks(self):
         from .qwen35_prefill import Qwen35Prefill

@@ -178,6 +178,9 @@ class DecodeSession:
     def generate(self, prompt_ids, max_new: int, use_graph: bool = True, eos=None) -> Generated:
         """Walk the prompt, then continue greedily for *max_new* tokens; one sync at each end.  *eos*: token ids
         that end the sequence; the tokens before the first of them are returned (``set_eos``)."""
+        return self._generate(prompt_ids, max_new, use_graph, eos, self._walk_prompt)
+
+    def _generate(self, prompt_ids, max_new: int, use_graph: bool, eos, take_prompt) -> Generated:
         if eos is not None:
             self.set_eos(eos)
         self.reset(prompt_ids)
@@ -188,7 +191,7 @@ class DecodeSession:
             self.capture()
         start, mid, end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
         start.record()
-        picked = self._take_prompt(max_new, use_graph, mid)
+        picked = take_prompt(max_new, use_graph, mid)
         self.run(max_new - picked, use_graph)      # step at position p writes token p+1
         end.record()
         torch.cuda.synchronize()
@@ -197,27 +200,31 @@ class DecodeSession:
         out = self.tokens[n_prompt: self.generated_end(n_prompt + max_new)].tolist()
         return Generated(out, mid.elapsed_time(end) / 1e3, start.elapsed_time(mid) / 1e3, n_prompt)
 
-    def _take_prompt(self, max_new: int, use_graph: bool, mid) -> int:
+    def _walk_prompt(self, max_new: int, use_graph: bool, mid) -> int:
         """The prompt's share of ``generate``: positions 0 .. n_prompt-2 (no sampling needed), then the event *mid*.
         Returns how many new tokens are picked already."""
         self.run(self.n_prompt - 1, use_graph)
         mid.record()
         return 0
 
-    def _prompt_in_chunks(self, chunks, max_new: int, mid) -> int:
-        """As ``_take_prompt`` with a chunk processor.  Where a new token is wanted the last prompt token goes through in the
+    def _chunk_prompt(self, max_new: int, use_graph: bool, mid) -> int:
+        """As ``_walk_prompt`` with a chunk processor.  Where a new token is wanted the last prompt token goes through in the
         chunk too, and the head on its row picks: a step for that token alone would read every weight a second time (a
         64-token request: 0.8 of 3.0 ms for Qwen3, 2.9 of 5.2 for MiniCPM3).  Two tokens are faster as two steps, and a
         session that records a trace takes the last one as a step."""
         if max_new < 1 or self.n_prompt < 3 or self.trace is not None:
-            chunks.run(self.n_prompt - 1, 0)
+            self._chunks().run(self.n_prompt - 1, 0)
             mid.record()
             return 0
-        last = chunks.run(self.n_prompt, 0, pick=True)
+        last = self._chunks().run(self.n_prompt, 0, pick=True)
         mid.record()
         if last is not None:
             self._pick_from(last)
         return 1
+
+    def _chunks(self):
+        """This session's chunk processor, made at its first use."""
+        raise NotImplementedError
 
     def _pick_from(self, hidden: int) -> None:
         """Final norm, head, pick and the advance of the position, from the last layer's output at address *hidden*: what a
