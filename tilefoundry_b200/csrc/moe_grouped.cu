@@ -172,8 +172,9 @@ __global__ void __launch_bounds__(1024) moe_batch_prepare_kernel(const MoeBatchP
     for (int a0 = 0; a0 < T * K; a0 += 1024) {
         for (int i = tid; i < 32 * 514; i += 1024) (&hist[0][0])[i] = 0;
         const int a = a0 + tid;
-        const bool live = a < T * K;
-        const int e = live ? int(p.indices[a]) : E + 1;        // (E + 1: a column nobody reads)
+        const long long named = a < T * K ? p.indices[a] : -1;
+        const bool live = named >= 0 && named < E;             // (an index that names no expert is on no list)
+        const int e = live ? int(named) : E + 1;               // (E + 1: a column nobody reads)
         __syncthreads();
         const unsigned same = __match_any_sync(0xffffffffu, e);
         const int rank = __popc(same & ((1u << lane) - 1u));
@@ -187,10 +188,11 @@ __global__ void __launch_bounds__(1024) moe_batch_prepare_kernel(const MoeBatchP
                 hist[w][tid] = short(n);
                 n += c;
             }
-            s_cnt[tid] = n;
+            s_cnt[tid] = min(n, T);                            // (a list holds T entries: a token names an expert once)
         }
         __syncthreads();
-        if (live) p.lists[size_t(e) * T + hist[warp][e] + rank] = ((a / K) << 8) | (a % K);
+        const int place = live ? hist[warp][e] + rank : T;
+        if (place < T) p.lists[size_t(e) * T + place] = ((a / K) << 8) | (a % K);
         __syncthreads();
     }
     // the shared expert takes every token, in slot K
