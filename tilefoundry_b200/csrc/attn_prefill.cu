@@ -18,6 +18,12 @@
 // rounding, which both share).  P overwrites S in place: columns 32c .. 32c+15 the hi terms of scores 32c .. 32c+31, the
 // next 16 their lo terms.  O is only rescaled when a row's maximum has grown by more than 8 (in log2), exact either way.
 //
+// The product meets every row of a V tile, so a row that a query must not see is more than a weight of zero (0 x Inf and
+// 0 x NaN are NaN).  In the one or two tiles that hold such rows the softmax warps look at V in shared memory first: rows past
+// the CTA's last token (a page's stale rows, later tokens) are zeroed; if a row of its own tokens is not finite, the CTA's
+// results are taken by a plain walk over the positions each query sees (slow_rows), as the decode kernels' are.  (The look
+// takes 16 conflict-free 16-byte reads a thread, under the tile's scores.)
+//
 // V as the second operand is [position][d] in shared memory, so N is its contiguous dimension: an MN-major descriptor
 // (64-element blocks 16 KB apart, groups of eight positions 1 KB apart).
 //
@@ -38,7 +44,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 struct PaTail {
     uint64_t q_full, k_full, v_full, k_empty, v_empty, s_full, p_full, o_done;
     uint32_t tmem_base;
-    volatile int aborted;
+    volatile int aborted, poisoned;
 };
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
@@ -206,6 +212,64 @@ __global__ void __launch_bounds__(256) mla_chunk_q_kernel(const MlaChunkParams p
     }
 }
 
+// ---- the plain walk -------------------------------------------------------------------------------------------------
+// 32 query rows from row0 of the tile, one after the other by a warp: f32 scores and sums over positions 0 .. the query's own,
+// nothing else is read.  Only for a tile whose own V rows are not all finite; four positions in flight.
+__device__ __forceinline__ float two_terms(uint16_t hi, uint16_t lo) {     // (of a value that is not finite, hi is the whole)
+    const float h = bf16_bits_to_f32(hi);
+    return (hi & 0x7f80u) == 0x7f80u ? h : h + bf16_bits_to_f32(lo);
+}
+template <int G, bool MLA>
+__device__ __noinline__ void slow_rows(const PrefillAttnParams& p, int first, int m0, int g, int row0, int lane) {
+    constexpr int OW = MLA ? 64 : PA_D, VPL = OW / 32, QPL = MLA ? 3 : 4;   // values a lane holds of an output, of a query
+    for (int r = row0; r < row0 + 32; ++r) {
+        const int tok = m0 + r / G, pos = first + tok, head = g * G + r % G;
+        if (tok >= p.m || pos >= p.max_ctx) continue;
+        float q[QPL], o[VPL], m = -INFINITY, l = 0.f;
+#pragma unroll
+        for (int i = 0; i < QPL; ++i)
+            q[i] = bf16_bits_to_f32(MLA ? p.qkv[(size_t(tok) * p.hq + head) * 96 + lane + 32 * i]
+                                        : p.qkv[(size_t(tok) * (p.hq + 2 * p.hkv) + head) * PA_D + lane + 32 * i]);
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) o[i] = 0.f;
+        for (int t0 = 0; t0 <= pos; t0 += 4) {
+            float s[4], v[4][VPL];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int t = min(t0 + j, pos);
+                const size_t row = size_t(p.block_table[t / p.page_size]) * p.page_size + t % p.page_size;
+                s[j] = 0.f;
+                if (MLA) {
+                    const size_t at = (size_t(t) * p.hkv + g) * 128 + lane;
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) s[j] = fmaf(q[i], two_terms(p.k_pool[at + 32 * i], p.v_pool[at + 32 * i]), s[j]);
+                    s[j] = fmaf(q[QPL - 1], bf16_bits_to_f32(p.lat_pool[row * 288 + 256 + lane]), s[j]);
+#pragma unroll
+                    for (int i = 0; i < VPL; ++i) v[j][i] = two_terms(p.k_pool[at + 64 + 32 * i], p.v_pool[at + 64 + 32 * i]);
+                } else {
+                    const size_t at = (row * p.hkv + g) * PA_D + lane;
+#pragma unroll
+                    for (int i = 0; i < QPL; ++i) s[j] = fmaf(q[i], bf16_bits_to_f32(p.k_pool[at + 32 * i]), s[j]);
+#pragma unroll
+                    for (int i = 0; i < VPL; ++i) v[j][i] = bf16_bits_to_f32(p.v_pool[at + 32 * i]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (t0 + j > pos) break;
+                const float sc = warp_sum(s[j]), nm = fmaxf(m, sc);
+                const float f = m == -INFINITY ? 0.f : __expf(m - nm), w = sc == -INFINITY ? 0.f : __expf(sc - nm);
+                l = l * f + w;
+#pragma unroll
+                for (int i = 0; i < VPL; ++i) o[i] = fmaf(w, v[j][i], o[i] * f);
+                m = nm;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) p.out[(size_t(tok) * p.hq + head) * OW + lane + 32 * i] = f32_to_bf16_bits(o[i] / l);
+    }
+}
+
 // ---- flash attention ----------------------------------------------------------------------------------------------
 // GQA form (G query heads per KV head): maps q, k, v.  Latent form (MLA, G = 1): a head's keys and values are expanded from
 // the latents to hi + lo bf16 terms beforehand, so a tile is K_hi | K_lo (64 wide each) and the rotary part shared by all
@@ -217,7 +281,7 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
                                                                      const __grid_constant__ CUtensorMap map_v,
                                                                      const __grid_constant__ CUtensorMap map_qr,
                                                                      const __grid_constant__ CUtensorMap map_kr,
-                                                                     const PrefillAttnParams p) {
+                                                                     const __grid_constant__ PrefillAttnParams p) {
     constexpr int TOK = 128 / G;                         // tokens of a query tile
     constexpr int OW = MLA ? 64 : PA_D;                  // width of a head's output
     constexpr int Q_BYTES = MLA ? PA_HALF + PA_HALF / 2 : PA_TILE, K_BYTES = MLA ? PA_TILE + PA_HALF / 2 : PA_TILE;
@@ -232,7 +296,7 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
         mbar_init(&t->q_full, 1); mbar_init(&t->k_full, 1); mbar_init(&t->v_full, 1);
         mbar_init(&t->k_empty, 1); mbar_init(&t->v_empty, 1); mbar_init(&t->s_full, 1);
         mbar_init(&t->p_full, 4); mbar_init(&t->o_done, 1);
-        t->aborted = 0;
+        t->aborted = t->poisoned = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {                                     // S / P: columns 0..127, O: 128..255
@@ -343,6 +407,26 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
         float m_run = -INFINITY, l_run = 0.f;            // maximum in log2 units
         bool ok = true;
         for (int i = 0; i < n_tiles; ++i) {
+            if ((i + 1) * PA_KV - 1 > first + m0) {      // V rows of this tile that some query must not see (uniform over the CTA)
+                ok = wait(&t->v_full, i & 1, 3u);
+                if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                const int pos = i * PA_KV + r;           // this thread's V row; its 16-byte pieces in the order that meets no bank twice
+                uint4* row = reinterpret_cast<uint4*>(vs + r * 128);
+                uint32_t most = 0;                       // the largest magnitudes of even and odd elements
+#pragma unroll
+                for (int c = 0; c < 16; ++c) {
+                    uint4* piece = row + (c >> 3) * (PA_HALF / 16) + ((c + r) & 7);
+                    if (pos > last) {
+                        *piece = make_uint4(0u, 0u, 0u, 0u);
+                    } else if (!MLA || c < 8) {          // (latent form: a value's first term tells)
+                        const uint4 u = *piece;
+                        most = __vmaxu2(__vmaxu2(__vmaxu2(most, u.x & 0x7fff7fffu), __vmaxu2(u.y & 0x7fff7fffu, u.z & 0x7fff7fffu)),
+                                        u.w & 0x7fff7fffu);
+                    }
+                }
+                if (pos > first + m0 && ((most & 0xffffu) >= 0x7f80u || (most >> 16) >= 0x7f80u)) t->poisoned = 1;
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the zeros, before the products read them
+            }
             ok = wait(&t->s_full, i & 1, 3u);
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -393,14 +477,15 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
                 l_run *= scale;
                 m_run = m_new;
             }
+            const float m_ref = m_run == -INFINITY ? 0.f : m_run;        // (no score above -infinity yet: no weight)
 #pragma unroll
             for (int c = 0; c < PA_KV / 32; ++c) {
                 uint32_t o[32];
                 float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
                 for (int j = 0; j < 32; j += 2) {
-                    const float a = ex2(fmaf(__uint_as_float(v[c][j]), kLog2e, -m_run));
-                    const float b = ex2(fmaf(__uint_as_float(v[c][j + 1]), kLog2e, -m_run));
+                    const float a = ex2(fmaf(__uint_as_float(v[c][j]), kLog2e, -m_ref));
+                    const float b = ex2(fmaf(__uint_as_float(v[c][j + 1]), kLog2e, -m_ref));
                     sum0 += a;
                     sum1 += b;
                     const uint32_t hi = pack2(a, b);
@@ -416,7 +501,10 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(&t->p_full)) : "memory");
         }
         if (ok) ok = wait(&t->o_done, (n_tiles - 1) & 1, 3u);
-        if (__all_sync(0xffffffffu, ok)) {
+        asm volatile("bar.sync 1, 128;" ::: "memory");   // every warp has looked at its V rows
+        if (t->poisoned) {
+            slow_rows<G, MLA>(p, first, m0, g, quad * 32, lane);
+        } else if (__all_sync(0xffffffffu, ok)) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const float inv = 1.f / l_run;
             uint16_t* dst = p.out + (size_t(tok) * p.hq + g * G + r % G) * OW;
@@ -514,6 +602,7 @@ cudaError_t mla_chunk_attn_launch(const MlaChunkParams& c, cudaStream_t stream, 
     if (e != cudaSuccess) return e;
     PrefillAttnParams p = {};
     p.pos_rows = c.pos_rows; p.block_table = c.block_table; p.out = c.out; p.status = c.status;
+    p.qkv = c.q; p.k_pool = const_cast<uint16_t*>(c.kv_hi); p.v_pool = const_cast<uint16_t*>(c.kv_lo); p.lat_pool = c.pool;
     p.m = c.m; p.hq = c.heads; p.hkv = c.heads; p.page_size = c.page_size; p.max_ctx = c.max_ctx;
     CUtensorMap m[5];
     const size_t ctx = size_t(c.first) + c.m, kvw = size_t(c.heads) * 128, qw = size_t(c.heads) * 96;

@@ -350,6 +350,7 @@ __global__ void __launch_bounds__(256) gated_chunk_attn_kernel(const GatedChunkP
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const float w = __shfl_sync(0xffffffffu, e[r], j);
+                if (k0 + j > first + m0 + (warp * 4 + r) / G) continue;      // (a later token's value is not multiplied: it may be NaN)
 #pragma unroll
                 for (int i = 0; i < EPL; ++i) o[r][i] = fmaf(w, v[i], o[r][i]);
             }

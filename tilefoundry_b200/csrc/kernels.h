@@ -402,7 +402,8 @@ struct PrefillAttnParams {
     uint16_t* qkv;               // bf16 [m][(hq + 2 hkv) * 128]; the q part is rewritten (normalised, rotated, scaled)
     const uint16_t *gamma_q, *gamma_k, *cos_table, *sin_table;
     const int* pos_rows;         // [m] consecutive positions
-    uint16_t *k_pool, *v_pool;   // [pages][page_size][hkv][128]
+    uint16_t *k_pool, *v_pool;   // [pages][page_size][hkv][128]; latent form: the hi and lo terms [position][head][keys | values]
+    const uint16_t* lat_pool;    // latent form: [pages][page_size][288]
     const int* block_table;
     uint16_t* out;               // bf16 [m][hq * 128]
     unsigned* status;
