@@ -484,14 +484,17 @@ __global__ void __launch_bounds__(kTopPThreads) top_p_pick_kernel(const TopPPara
     const int span = gridDim.x * kTopPThreads;
     for (int i0 = blockIdx.x * kTopPThreads + warp * 32; i0 < p.vocab; i0 += 4 * span) {     // four tokens per lane at a time
         float logit[4], est[4], top = -INFINITY;
+        bool in[4];                                            // (in the nucleus: an infinite estimate does not tell)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int i = i0 + q * span + lane;
             est[q] = -INFINITY;
             logit[q] = 0.f;
+            in[q] = false;
             if (i < p.vocab) {
                 const uint16_t b = p.logits[i];
                 if (bf16_key(b) >= tau) {
+                    in[q] = true;
                     logit[q] = __fdiv_rn(bf16_bits_to_f32(b), p.temperature);
                     est[q] = logit[q] + gumbel_estimate(p.seed, step, i);
                 }
@@ -499,10 +502,11 @@ __global__ void __launch_bounds__(kTopPThreads) top_p_pick_kernel(const TopPPara
             top = fmaxf(top, est[q]);
         }
         top = warp_max(top);
-        const float margin = top - 0.01f - 1e-6f * fabsf(top);
+        // (all tokens at an infinite top are at the margin: the lowest index of them is the pick)
+        const float margin = fabsf(top) == INFINITY ? top : top - 0.01f - 1e-6f * fabsf(top);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-            if (est[q] != -INFINITY && est[q] >= margin) {
+            if (in[q] && est[q] >= margin) {
                 const int i = i0 + q * span + lane;
                 take(logit[q] + gumbel_variate(p.seed, step, i), i);
             }
