@@ -204,3 +204,33 @@ def test_nucleus_sampling_rejects_bad_arguments(so):
     assert call(a(vocab=0)) == EINVAL
     assert call(a(n_eos=2)) == EINVAL and call(a(n_eos=2, eos_ids=P)) == EINVAL      # end ids come with their latch
     assert call(a(n_eos=17, eos_ids=P, stop_at=P)) == EINVAL
+
+
+def test_qwen35_chunks_refuse_shapes_and_layers_their_kernels_do_not_hold(so):
+    step = dict(n_layers=1, hidden=256, vocab=1000, hk=2, hv=4, dk=128, dv=128, conv_width=4, hq=4, hkv=2, d=128, rotary_dim=64, experts=16,
+                top_k=4, inter=256, shared_inter=256, conv_state_stride=3 * 1024, page_size=64, table_len=4, max_ctx=256, table=P,
+                block_table=P, cos_table=P, sin_table=P)
+    supported = lambda **kw: so.tfb_qwen35_prefill_supported(C.byref(lib.Qwen35StepArgs(**{**step, **kw})))
+    assert supported() == 1 and supported(hk=1, hv=2) == 1
+    assert supported(hk=1, hv=3) == 0                       # a row of the projection would start between 8-byte boundaries
+    assert supported(hk=1, hv=1) == 0 and supported(rotary_dim=0) == 0 and supported(hv=3) == 0
+    buffers = ("ids", "pos_rows", "hidden", "attended", "normed", "norm16", "proj", "mixed", "out16", "qk", "v", "read", "gates", "logits",
+               "indices", "weights", "shared_gate", "inner", "y", "counts", "lists", "status")
+
+    def call(layer=None, step_kw=None, **kw):
+        layer = layer or {}
+        fields = {n: layer.get(n, P) for n, _ in lib.Qwen35Layer._fields_ if n not in ("kind", "reserved")}
+        layers = (lib.Qwen35Layer * 1)(lib.Qwen35Layer(kind=layer.get("kind", 0), **fields))
+        s = lib.Qwen35StepArgs(layers=layers, **{**step, **(step_kw or {})})
+        return so.tfb_qwen35_prefill_chunk(C.byref(lib.Qwen35PrefillArgs(step=C.pointer(s), **{**{n: P for n in buffers}, "m": 4, **kw})), None)
+    for n in buffers:
+        assert call(**{n: None}) == EINVAL, n
+    for n in ("hidden", "attended", "normed", "norm16", "proj", "mixed", "out16", "qk", "v", "read"):
+        assert call(**{n: ODD}) == EALIGN, n
+    assert call(m=1) == EINVAL and call(m=4097) == EINVAL and call(step_kw={"hk": 1, "hv": 3}) == EINVAL
+    assert call(step_kw={"table_len": 3}) == ECAPACITY and call(step_kw={"page_size": 48, "table_len": 6}) == EINVAL
+    assert call(step_kw={"conv_state_stride": 3 * 1024 - 1}) == EINVAL
+    for kind, names in ((0, ("conv_w", "a_log", "dt_bias", "gamma_gdn", "conv_state", "state")), (1, ("gamma_q", "gamma_k", "k_pool", "v_pool"))):
+        for n in names + ("gamma_in", "w_in", "w_out", "gamma_post", "w_router", "w_gate", "w_up", "w_down", "w_shared_gate"):
+            assert call({"kind": kind, n: None}) == EINVAL, (kind, n)
+    assert call({"gamma_gdn": ODD}) == EALIGN and call({"kind": 1, "k_pool": ODD}) == EALIGN and call({"w_in": ODD}) == EALIGN

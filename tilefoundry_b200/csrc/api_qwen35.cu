@@ -344,6 +344,28 @@ int tfb_qwen35_prefill_chunk(const tfb_qwen35_prefill_args* a, tfb_stream_t stre
     TFB_REQUIRE(a->hidden && a->attended && a->normed && a->norm16 && a->proj && a->mixed && a->out16 && a->qk && a->v && a->read &&
                     a->gates && a->logits && a->indices && a->weights && a->shared_gate && a->inner && a->y && a->counts && a->lists && a->status,
                 TFB_EINVAL);
+    // everything is checked before anything is queued: what the step's entries check per layer, and what the chunk's kernels
+    // read 8 or 16 bytes at a time
+    TFB_REQUIRE(s->page_size > 0 && s->page_size % 64 == 0 && s->max_ctx > 0, TFB_EINVAL);
+    TFB_REQUIRE((long long)s->page_size * s->table_len >= s->max_ctx, TFB_ECAPACITY);
+    TFB_REQUIRE(s->conv_state_stride >= 3ull * (2ull * s->hk * s->dk + uint64_t(s->hv) * s->dv), TFB_EINVAL);
+    for (const void* q : {(const void*)a->hidden, (const void*)a->attended, (const void*)a->normed, (const void*)a->norm16,
+                          (const void*)a->proj, (const void*)a->mixed, (const void*)a->out16, (const void*)a->qk, (const void*)a->v,
+                          (const void*)a->read})
+        TFB_REQUIRE(aligned16(q), TFB_EALIGN);
+    for (int l = 0; l < s->n_layers; ++l) {
+        const tfb_qwen35_layer& L = s->layers[l];
+        TFB_REQUIRE(L.gamma_in && L.w_in && L.w_out && L.gamma_post && L.w_router && L.w_gate && L.w_up && L.w_down && L.w_shared_gate &&
+                        L.w_shared_up && L.w_shared_down, TFB_EINVAL);
+        TFB_REQUIRE(aligned16(L.w_in) && aligned16(L.w_out), TFB_EALIGN);
+        if (L.kind == 0) {
+            TFB_REQUIRE(L.conv_w && L.a_log && L.dt_bias && L.gamma_gdn && L.conv_state && L.state, TFB_EINVAL);
+            TFB_REQUIRE(aligned16(L.gamma_gdn), TFB_EALIGN);
+        } else {
+            TFB_REQUIRE(L.gamma_q && L.gamma_k && L.k_pool && L.v_pool, TFB_EINVAL);
+            TFB_REQUIRE(aligned16(L.k_pool) && aligned16(L.v_pool), TFB_EALIGN);
+        }
+    }
     const bool pdl = a->pdl != 0;
     const int M = a->m, H = s->hidden, KEY = s->hk * s->dk, VAL = s->hv * s->dv, CONV = 2 * KEY + VAL;
     const int N_GDN = CONV + VAL + 2 * s->hv, QD = s->hq * s->d, N_ATT = 2 * QD + 2 * s->hkv * s->d;

@@ -391,7 +391,8 @@ cudaError_t add_norm_rows_launch(const float* x, const uint16_t* y, const float*
 }
 
 bool gdn_chunk_supported(int hk, int hv, int dk, int dv, int width) {
-    return dk == 128 && dv == 128 && width == 4 && hk > 0 && hv % hk == 0 && hv <= 256;
+    // (an even hv: a token's row of the projection, with the two scalars per value head at its end, is read 8 bytes at a time)
+    return dk == 128 && dv == 128 && width == 4 && hk > 0 && hv > 0 && hv % hk == 0 && hv % 2 == 0 && hv <= 256;
 }
 cudaError_t gdn_chunk_launch(const GdnChunkParams& p, cudaStream_t stream, bool pdl) {
     cudaError_t e = launch_kernel(gdn_chunk_prep_kernel, dim3(p.m, (2 * p.hk + p.hv + 7) / 8), dim3(256), 0, stream, pdl, p);
@@ -401,7 +402,8 @@ cudaError_t gdn_chunk_launch(const GdnChunkParams& p, cudaStream_t stream, bool 
 }
 
 bool gated_chunk_supported(int hq, int hkv, int d, int rotary_dim) {
-    return (d == 128 || d == 256) && hkv > 0 && hq % hkv == 0 && 32 % (hq / hkv) == 0 && rotary_dim % 64 == 0 && rotary_dim <= d;
+    return (d == 128 || d == 256) && hkv > 0 && hq > 0 && hq % hkv == 0 && 32 % (hq / hkv) == 0 && rotary_dim > 0 &&
+           rotary_dim % 64 == 0 && rotary_dim <= d;
 }
 cudaError_t gated_chunk_launch(const GatedChunkParams& p, int d, cudaStream_t stream, bool pdl) {
     return d == 256 ? gated_launch<256>(p, stream, pdl) : gated_launch<128>(p, stream, pdl);
