@@ -206,6 +206,43 @@ def test_nucleus_sampling_rejects_bad_arguments(so):
     assert call(a(n_eos=17, eos_ids=P, stop_at=P)) == EINVAL
 
 
+def test_prompt_chunks_refuse_what_their_layers_lack(so):
+    """Every pointer, alignment and capacity that a chunk's launches rely on is checked before the first of them."""
+    qwen = dict(n_layers=1, m=4, hidden=256, hq=4, hkv=2, d=128, inter=256, pdl=0, eps=1e-6, scale=0.1, vocab=1000, w_embed=P, cos_table=P,
+                sin_table=P, max_pos=256, page_size=64, table_len=4, max_ctx=256, block_table=P, ids=P, pos_rows=P, hidden_buf=P,
+                norm_buf=P, qkv_buf=P, attn_buf=P, act_buf=P, status=P)
+    mini = dict(n_layers=1, m=4, hidden=256, heads=4, q_lora=256, kv_lora=256, nope=64, rope=32, v=64, inter=256, vocab=1000, eps=1e-6,
+                lora_eps=1e-6, scale=0.1, embed_scale=1.0, residual_scale=1.0, pdl=0, w_embed=P, cos_table=P, sin_table=P, max_pos=256,
+                page_size=64, table_len=4, max_ctx=256, block_table=P, ids=P, pos_rows=P, hidden_buf=P, norm_buf=P, qkv_a_buf=P,
+                attn_buf=P, act_buf=P, status=P, qa_buf=P, lat_buf=P, q_buf=P, kv_hi_buf=P, kv_lo_buf=P, first=0)
+    up = P + 2 * 256 * 256                                  # right behind the gate rows
+
+    def call(entry, args, layer_type, base, layer, **kw):
+        fields = {n: layer.get(n, P) for n, _ in layer_type._fields_}
+        layers = (layer_type * 1)(layer_type(**fields))
+        return entry(C.byref(args(layers=layers, **{**base, **kw})), None)
+    qcall = lambda layer={}, **kw: call(so.tfb_qwen3_prefill_chunk, lib.Qwen3PrefillArgs, lib.Qwen3BatchLayer, qwen, layer, **kw)
+    mcall = lambda layer={}, **kw: call(so.tfb_minicpm3_prefill_chunk, lib.MiniCPM3PrefillArgs, lib.MiniCPM3Layer, mini, {"w_up": up, **layer}, **kw)
+    for n in ("gamma_in", "w_qkv", "gamma_q", "gamma_k", "w_o", "gamma_post", "w_gate_up", "w_down", "k_pool", "v_pool"):
+        assert qcall({n: None}) == EINVAL, n
+    for n in ("w_qkv", "w_o", "w_gate_up", "w_down", "k_pool", "v_pool"):
+        assert qcall({n: ODD}) == EALIGN, n
+    for n in ("norm_buf", "qkv_buf", "attn_buf", "act_buf"):
+        assert qcall(**{n: ODD}) == EALIGN, n
+    assert qcall(max_ctx=0) == EINVAL and qcall(table_len=3) == ECAPACITY and qcall(max_pos=255) == ECAPACITY
+    for n in ("gamma_in", "w_qkv_a", "gamma_q_a", "w_q_b", "gamma_kv_a", "w_kv_b", "w_o", "gamma_post", "w_gate", "w_up", "w_down", "k_pool"):
+        assert mcall({n: None}) == EINVAL, n
+    for n in ("w_qkv_a", "w_q_b", "w_kv_b", "w_o", "w_down", "k_pool"):
+        assert mcall({n: ODD}) == EALIGN, n
+    for n in ("norm_buf", "qkv_a_buf", "attn_buf", "act_buf", "qa_buf", "lat_buf", "q_buf", "kv_hi_buf", "kv_lo_buf"):
+        assert mcall(**{n: ODD}) == EALIGN, n
+    assert mcall(page_size=0) == EINVAL and mcall(table_len=0) == EINVAL
+    assert mcall(table_len=3) == ECAPACITY and mcall(max_pos=255) == ECAPACITY and mcall(first=253) == ECAPACITY
+    # the form of up to 32 tokens
+    small = dict(qa_buf=None, q_lat_buf=P, q_rope_buf=P, part_o=P, part_ml=P)
+    assert mcall({"k_pool": None}, **small) == EINVAL and mcall(m=33, **small) == EINVAL and mcall(table_len=3, **small) == ECAPACITY
+
+
 def test_qwen35_chunks_refuse_shapes_and_layers_their_kernels_do_not_hold(so):
     step = dict(n_layers=1, hidden=256, vocab=1000, hk=2, hv=4, dk=128, dv=128, conv_width=4, hq=4, hkv=2, d=128, rotary_dim=64, experts=16,
                 top_k=4, inter=256, shared_inter=256, conv_state_stride=3 * 1024, page_size=64, table_len=4, max_ctx=256, table=P,

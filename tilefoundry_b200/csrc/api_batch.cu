@@ -105,7 +105,16 @@ int tfb_qwen3_prefill_chunk(const tfb_qwen3_prefill_args* a, tfb_stream_t stream
     TFB_REQUIRE(a->status && (tc_attn || (a->part_o && a->part_ml && a->counters)), TFB_EINVAL);
     TFB_REQUIRE(!tc_attn || (aligned16(a->qkv_buf) && aligned16(a->attn_buf)), TFB_EALIGN);
     TFB_REQUIRE(a->hidden % 64 == 0 && a->inter % 64 == 0 && (a->hq * a->d) % 64 == 0, TFB_EINVAL);
+    TFB_REQUIRE(a->max_ctx > 0, TFB_EINVAL);
     TFB_REQUIRE((long long)a->page_size * a->table_len >= a->max_ctx && a->max_pos >= a->max_ctx, TFB_ECAPACITY);
+    TFB_REQUIRE(aligned16(a->norm_buf) && aligned16(a->attn_buf) && aligned16(a->act_buf), TFB_EALIGN);
+    for (int l = 0; l < a->n_layers; ++l) {                // (the launches below take the layers as they are)
+        const tfb_qwen3_batch_layer& L = a->layers[l];
+        TFB_REQUIRE(L.gamma_in && L.w_qkv && L.gamma_q && L.gamma_k && L.w_o && L.gamma_post && L.w_gate_up && L.w_down && L.k_pool &&
+                        L.v_pool, TFB_EINVAL);
+        TFB_REQUIRE(aligned16(L.w_qkv) && aligned16(L.w_o) && aligned16(L.w_gate_up) && aligned16(L.w_down) && aligned16(L.k_pool) &&
+                        aligned16(L.v_pool), TFB_EALIGN);
+    }
     const bool pdl = a->pdl != 0;
     const int M = a->m, H = a->hidden, QP = a->hq * a->d, KVP = a->hkv * a->d, I = a->inter;
     const int NQKV = QP + 2 * KVP;

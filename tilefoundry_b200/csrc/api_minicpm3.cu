@@ -84,6 +84,19 @@ int tfb_minicpm3_prefill_chunk(const tfb_minicpm3_prefill_args* a, tfb_stream_t 
     TFB_REQUIRE(!wide || a->first + a->m <= a->max_ctx, TFB_ECAPACITY);
     TFB_REQUIRE(a->hidden % 64 == 0 && a->inter % 64 == 0 && (a->heads * a->v) % 64 == 0, TFB_EINVAL);
     TFB_REQUIRE(tfb::mla_latent_supported(a->heads, a->q_lora, a->kv_lora, a->nope, a->rope, a->v, a->max_ctx), TFB_EINVAL);
+    TFB_REQUIRE(a->page_size > 0 && a->table_len > 0, TFB_EINVAL);
+    TFB_REQUIRE((long long)a->page_size * a->table_len >= a->max_ctx && a->max_pos >= a->max_ctx, TFB_ECAPACITY);
+    TFB_REQUIRE(aligned16(a->norm_buf) && aligned16(a->qkv_a_buf) && aligned16(a->attn_buf) && aligned16(a->act_buf), TFB_EALIGN);
+    TFB_REQUIRE(!wide || (aligned16(a->qa_buf) && aligned16(a->lat_buf) && aligned16(a->q_buf) && aligned16(a->kv_hi_buf) &&
+                          aligned16(a->kv_lo_buf)), TFB_EALIGN);
+    for (int l = 0; l < a->n_layers; ++l) {                // (the launches below take the layers as they are)
+        const tfb_minicpm3_layer& L = a->layers[l];
+        TFB_REQUIRE(L.gamma_in && L.w_qkv_a && L.gamma_q_a && L.w_q_b && L.gamma_kv_a && L.w_kv_b && L.w_o && L.gamma_post && L.w_gate &&
+                        L.w_down && L.k_pool, TFB_EINVAL);
+        TFB_REQUIRE(static_cast<const uint16_t*>(L.w_up) == static_cast<const uint16_t*>(L.w_gate) + size_t(a->inter) * a->hidden, TFB_EINVAL);
+        TFB_REQUIRE(aligned16(L.w_qkv_a) && aligned16(L.w_q_b) && aligned16(L.w_kv_b) && aligned16(L.w_o) && aligned16(L.w_gate) &&
+                        aligned16(L.w_down) && aligned16(L.k_pool), TFB_EALIGN);
+    }
     const bool pdl = a->pdl != 0;
     const int M = a->m, H = a->hidden, I = a->inter, NH = a->heads;
     const int NA = a->q_lora + a->kv_lora + a->rope, NO = NH * a->v;
@@ -109,7 +122,6 @@ int tfb_minicpm3_prefill_chunk(const tfb_minicpm3_prefill_args* a, tfb_stream_t 
     if (e != cudaSuccess) return fail_launch(e);
     for (int l = 0; l < a->n_layers; ++l) {
         const tfb_minicpm3_layer& L = a->layers[l];
-        TFB_REQUIRE(static_cast<const uint16_t*>(L.w_up) == static_cast<const uint16_t*>(L.w_gate) + size_t(I) * H, TFB_EINVAL);
         int rc = norm(L.gamma_in);
         if (rc) return rc;
         if ((rc = project(L.w_qkv_a, nrm, nullptr, qkv_a, NA, H, false))) return rc;
