@@ -77,6 +77,13 @@ def test_token_tiles_and_splits(dev, m, n, k):
     assert ((y.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -7 * prod.abs() + 1e-6).all()
 
 
+# either side of the lines between split counts: clusters of four and three, two splits on a shared SM, halves of 128 tokens
+@pytest.mark.parametrize("m,n,k", [(129, 4224, 512), (129, 4352, 512), (200, 5632, 320), (200, 5760, 320), (192, 2304, 512), (193, 2304, 512),
+                                   (33, 9472, 256), (128, 9600, 256), (64, 4864, 512), (100, 2304, 1024), (32, 4736, 512), (500, 2176, 320)])
+def test_lines_between_split_counts(dev, m, n, k):
+    test_token_tiles_and_splits(dev, m, n, k)
+
+
 @pytest.mark.parametrize("experts,top_k", [(5, 5), (72, 10), (128, 32), (256, 8)])
 def test_selection_orders_ties_zeros_and_infinities(dev, experts, top_k):
     from tilefoundry_b200 import lib

@@ -13,7 +13,7 @@
 //
 // Roles in a CTA of 6 warps: warp 0 (one lane) issues TMA loads; warp 1 allocates tensor memory and (one lane)
 // issues the MMAs, four per stage (K = 16 each), releasing a stage with tcgen05.commit; warps 2-5 read the
-// accumulator back (tcgen05.ld, one TMEM lane quadrant each) and write it out.  K is split over the 1, 2, 4 or 8
+// accumulator back (tcgen05.ld, one TMEM lane quadrant each) and write it out.  K is split over the 1, 2, 3, 4 or 8
 // CTAs of a thread-block cluster so that a 2048 x 2048 projection (16 row tiles) still reaches most SMs.  The
 // splits' f32 partials never leave the chip: every CTA parks its 128 x BN tile in its own shared memory, and
 // after a cluster barrier CTA c adds, in fixed split order (deterministic), token rows c, c + S, ... from all S CTAs through
@@ -35,6 +35,7 @@
 #include "launch.h"
 #include "tc.cuh"
 
+#include <algorithm>
 #include <cuda.h>
 
 namespace tfb {
@@ -273,26 +274,41 @@ __global__ void __launch_bounds__(TC_THREADS, TcShape<BN>::kCtas) gemm_tc_kernel
     if (p.splits > 1) cluster_sync_all();                               // nobody leaves while its tile is still being read
 }
 
-// K splits = CTAs of one cluster: the largest power of two that keeps the grid within the CTAs the chip holds at once, at
-// most 8 (the portable cluster size), and at most 4 where a CTA takes an SM to itself (clusters of 8 SMs do not all find
-// room at the same time: 2048 x 2048 at 193 tokens took 19 us with 8, 10.8 us with 4).
+// K splits = CTAs of one cluster, a power of two (or three, below): as many as keep the grid within `resident` CTAs, at most
+// `most` (8 is the portable cluster size).
 static int splits_for_tiles(int tiles, int k, int resident, int most) {
     int splits = 1;
     while (splits < most && tiles * splits * 2 <= resident && (k / TC_BK) % (splits * 2) == 0) splits *= 2;
     return splits;
 }
-int gemm_tc_splits(int n, int k) { return splits_for_tiles((n + TC_BM - 1) / TC_BM, k, sm_count(), 8); }
-int gemm_tc_splits_swiglu(int n, int k) { return splits_for_tiles((n + 63) / 64, k, sm_count(), 8); }
-// 129 .. 256 tokens as two tiles of 128 beside one another, where the weight tiles are few: @HALVES@
-static bool two_halves(int m, int tiles) { return m > 128 && m <= 256 && 8 * tiles <= sm_count(); }
+// Up to 32 tokens two CTAs share an SM and the weight stream is all there is: up to 8 splits within two CTAs per SM (4096 x
+// 2048: 7.9 us, with four splits 8.1; 6400 gate/up pairs x 2560: 16.1, unsplit 16.8).
+int gemm_tc_splits(int n, int k) { return splits_for_tiles((n + TC_BM - 1) / TC_BM, k, 2 * sm_count(), 8); }
+int gemm_tc_splits_swiglu(int n, int k) { return splits_for_tiles((n + 63) / 64, k, 2 * sm_count(), 8); }
+// More than 192 of up to 256 tokens as two tiles of 128 beside one another, where the weight tiles are few: two CTAs share
+// an SM again (256 tokens: 2304 x 2560 12.2 us, as one tile 13.4; 2048 x 2048 11.1, 12.2; 193: 11.4, 12.1 and 10.8, 11.0).
+// With fewer tokens in the second tile the first is not worth its weights twice (129: 11.5, 10.7 and 10.8, 9.6).  More weight
+// tiles fill the chip as they are (2560 x 2560, 20 tiles, 256 tokens: 15.4 us as halves, 13.4 as one).
+static bool two_halves(int m, int tiles) { return m > 192 && m <= 256 && 8 * tiles <= sm_count(); }
 int gemm_tc_splits_for(int m, int n, int k, bool swiglu) {
     const int tiles = swiglu ? (n + 63) / 64 : (n + TC_BM - 1) / TC_BM;
     if (two_halves(m, tiles)) return splits_for_tiles(2 * tiles, k, sm_count(), 4);
     if (m > 128) {
-        const int all = tiles * ((m + 255) / 256), s = splits_for_tiles(all, k, sm_count(), 4);
-        return s == 2 && 3 * all <= sm_count() ? 3 : s;      // (K steps that do not divide are dealt as evenly as they go)
+        // A CTA takes an SM to itself: at most 4 splits, and 4 or 3 only where that many clusters find room at the same time --
+        // of 148 SMs 33 clusters of four and 45 of three do, one more and they run in two waves (K 2048, 256 tokens, four: 33
+        // tiles 13.7 us, 34 24.6; three: 45 tiles 16.3, 46 28.3; 2048 x 2048 at 193 tokens took 19 us with clusters of 8).
+        // Nine tenths of the SMs keep clear of both.  Three, where four is too many or does not divide K, against two (K steps
+        // are dealt as evenly as they go): 40 tiles, K 2560, 256 tokens 16.2 us, 20.2.
+        const int all = tiles * ((m + 255) / 256), room = sm_count() * 9 / 10, s = splits_for_tiles(all, k, sm_count(), 4);
+        if (s == 4 && 4 * all <= room) return 4;
+        return s >= 2 && 3 * all <= room ? 3 : std::min(s, 2);
     }
-    return splits_for_tiles(tiles, k, sm_count(), 8);
+    if (m <= 32) return splits_for_tiles(tiles, k, 2 * sm_count(), 8);
+    // 33 .. 128 tokens: two CTAs share an SM, worth it up to 4 splits (6400 gate/up pairs x 2560, 128 tokens: two splits 20.1 us,
+    // unsplit 23.8; 8192 x 2048: four 13.5, two 15.9; 97 .. 148 tiles at 64 tokens 1 to 2 % slower, at 96 3 to 6 % faster);
+    // 8 only within one CTA per SM (4096 x 2048, 128 tokens: eight 12.4 us, four 11.6).
+    const int s = splits_for_tiles(tiles, k, 2 * sm_count(), 4);
+    return s == 4 ? std::max(s, splits_for_tiles(tiles, k, sm_count(), 8)) : s;
 }
 
 // Weights [rows][K], boxes of 64 elements x box_rows of each half (halves = 2: gate rows, then up rows).
