@@ -281,10 +281,18 @@ static int splits_for_tiles(int tiles, int k, int resident, int most) {
     while (splits < most && tiles * splits * 2 <= resident && (k / TC_BK) % (splits * 2) == 0) splits *= 2;
     return splits;
 }
-// Up to 32 tokens two CTAs share an SM and the weight stream is all there is: up to 8 splits within two CTAs per SM (4096 x
-// 2048: 7.9 us, with four splits 8.1; 6400 gate/up pairs x 2560: 16.1, unsplit 16.8).
-int gemm_tc_splits(int n, int k) { return splits_for_tiles((n + TC_BM - 1) / TC_BM, k, 2 * sm_count(), 8); }
-int gemm_tc_splits_swiglu(int n, int k) { return splits_for_tiles((n + 63) / 64, k, 2 * sm_count(), 8); }
+// Up to 128 tokens two CTAs share an SM, worth it up to 4 splits (6400 gate/up pairs x 2560, 128 tokens: two splits 20.1 us,
+// unsplit 23.8; 8192 x 2048: four 13.5, two 15.9; the MiniCPM3 prompt of 128 tokens 7.1 ms, one CTA per SM 7.6); 8 only within
+// one CTA per SM (4096 x 2048, 128 tokens: eight 12.4 us, four 11.6; alone and with 32 tokens eight are 0.3 us faster, but the
+// 32-sequence step of Qwen3 is 2.70 ms with them, 2.63 with four).  Up to 32 tokens a share of less than 20 blocks of K is not
+// worth a second CTA on an SM (6144 gate/up pairs x 2048: two splits 14.7 us, unsplit 14.4; 6400 x 2560: 16.1, 16.7).
+static int splits_two_per_sm(int tiles, int k, bool few) {
+    const int sms = sm_count(), s = splits_for_tiles(tiles, k, 2 * sms, 4);
+    if (s == 2 && few && 2 * tiles > sms && k < 40 * TC_BK) return 1;
+    return s == 4 ? std::max(s, splits_for_tiles(tiles, k, sms, 8)) : s;
+}
+int gemm_tc_splits(int n, int k) { return splits_two_per_sm((n + TC_BM - 1) / TC_BM, k, true); }
+int gemm_tc_splits_swiglu(int n, int k) { return splits_two_per_sm((n + 63) / 64, k, true); }
 // More than 192 of up to 256 tokens as two tiles of 128 beside one another, where the weight tiles are few: two CTAs share
 // an SM again (256 tokens: 2304 x 2560 12.2 us, as one tile 13.4; 2048 x 2048 11.1, 12.2; 193: 11.4, 12.1 and 10.8, 11.0).
 // With fewer tokens in the second tile the first is not worth its weights twice (129: 11.5, 10.7 and 10.8, 9.6).  More weight
@@ -303,12 +311,7 @@ int gemm_tc_splits_for(int m, int n, int k, bool swiglu) {
         if (s == 4 && 4 * all <= room) return 4;
         return s >= 2 && 3 * all <= room ? 3 : std::min(s, 2);
     }
-    if (m <= 32) return splits_for_tiles(tiles, k, 2 * sm_count(), 8);
-    // 33 .. 128 tokens: two CTAs share an SM, worth it up to 4 splits (6400 gate/up pairs x 2560, 128 tokens: two splits 20.1 us,
-    // unsplit 23.8; 8192 x 2048: four 13.5, two 15.9; 97 .. 148 tiles at 64 tokens 1 to 2 % slower, at 96 3 to 6 % faster);
-    // 8 only within one CTA per SM (4096 x 2048, 128 tokens: eight 12.4 us, four 11.6).
-    const int s = splits_for_tiles(tiles, k, 2 * sm_count(), 4);
-    return s == 4 ? std::max(s, splits_for_tiles(tiles, k, sm_count(), 8)) : s;
+    return splits_two_per_sm(tiles, k, m <= 32);
 }
 
 // Weights [rows][K], boxes of 64 elements x box_rows of each half (halves = 2: gate rows, then up rows).
