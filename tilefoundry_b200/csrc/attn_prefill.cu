@@ -19,10 +19,11 @@
 // next 16 their lo terms.  O is only rescaled when a row's maximum has grown by more than 8 (in log2), exact either way.
 //
 // The product meets every row of a V tile, so a row that a query must not see is more than a weight of zero (0 x Inf and
-// 0 x NaN are NaN).  In the one or two tiles that hold such rows the softmax warps look at V in shared memory first: rows past
-// the CTA's last token (a page's stale rows, later tokens) are zeroed; if a row of its own tokens is not finite, the CTA's
-// results are taken by a plain walk over the positions each query sees (slow_rows), as the decode kernels' are.  (The look
-// takes 16 conflict-free 16-byte reads a thread, under the tile's scores.)
+// 0 x NaN are NaN).  Rows past the chunk (a page's stale rows) are zeroed in shared memory by the requesting warp
+// while the softmax runs (by the softmax warps themselves it cost 1.5 us a layer); a warp one of whose
+// results is not finite -- a later token of the tile may have done that, or an earlier one rightly -- takes its
+// rows again by a plain walk over the positions each query sees (slow_rows), as the decode kernels take them.  (Looking through
+// the V tile for such values instead cost 1.6 us a layer.)
 //
 // V as the second operand is [position][d] in shared memory, so N is its contiguous dimension: an MN-major descriptor
 // (64-element blocks 16 KB apart, groups of eight positions 1 KB apart).
@@ -42,9 +43,9 @@ constexpr int PA_TILE = 2 * PA_HALF;
 constexpr float kLog2e = 1.4426950408889634f;
 
 struct PaTail {
-    uint64_t q_full, k_full, v_full, k_empty, v_empty, s_full, p_full, o_done;
+    uint64_t q_full, k_full, v_full, v_clean, k_empty, v_empty, s_full, p_full, o_done;
     uint32_t tmem_base;
-    volatile int aborted, poisoned;
+    volatile int aborted;
 };
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(256) mla_chunk_q_kernel(const MlaChunkParams p
 
 // ---- the plain walk -------------------------------------------------------------------------------------------------
 // 32 query rows from row0 of the tile, one after the other by a warp: f32 scores and sums over positions 0 .. the query's own,
-// nothing else is read.  Only for a tile whose own V rows are not all finite; four positions in flight.
+// nothing else is read.  Only where a result was not finite; four positions in flight.
 __device__ __forceinline__ float two_terms(uint16_t hi, uint16_t lo) {     // (of a value that is not finite, hi is the whole)
     const float h = bf16_bits_to_f32(hi);
     return (hi & 0x7f80u) == 0x7f80u ? h : h + bf16_bits_to_f32(lo);
@@ -293,10 +294,10 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
     const int m0 = (gridDim.y - 1 - blockIdx.y) * TOK, g = blockIdx.x;   // the longest tiles of every KV head first
 
     if (threadIdx.x == 0) {
-        mbar_init(&t->q_full, 1); mbar_init(&t->k_full, 1); mbar_init(&t->v_full, 1);
+        mbar_init(&t->q_full, 1); mbar_init(&t->k_full, 1); mbar_init(&t->v_full, 1); mbar_init(&t->v_clean, 1);
         mbar_init(&t->k_empty, 1); mbar_init(&t->v_empty, 1); mbar_init(&t->s_full, 1);
         mbar_init(&t->p_full, 4); mbar_init(&t->o_done, 1);
-        t->aborted = t->poisoned = 0;
+        t->aborted = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {                                     // S / P: columns 0..127, O: 128..255
@@ -313,6 +314,8 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
     const int first = p.pos_rows[0];                     // positions of a chunk are consecutive
     const int last = min(first + min(m0 + TOK, p.m) - 1, p.max_ctx - 1);
     const int n_tiles = first < 0 ? 0 : (last + 1 + PA_KV - 1) / PA_KV;
+    // V rows of the last tile past the chunk, whatever the pages hold there (the latent form's tiles end with the chunk: zeros)
+    const int stale = MLA || n_tiles == 0 ? 0 : max(n_tiles * PA_KV - min(first + p.m, p.max_ctx), 0);
 
     auto wait = [&](uint64_t* bar, uint32_t parity, unsigned role) -> bool {
         if (t->aborted) return false;
@@ -358,6 +361,17 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
                 if (MLA) load_mla(vs, &t->v_full, i, false); else load(vs, &map_v, &t->v_full, i);
             }
         }
+        __syncwarp();
+        if (stale > 0) {                                 // zeros, under the softmax
+            const bool ok = wait(&t->v_full, (n_tiles - 1) & 1, 1u);
+            if (__all_sync(0xffffffffu, ok)) {
+                for (int c = lane; c < stale * 16; c += 32)
+                    reinterpret_cast<uint4*>(vs + (c & 8 ? PA_HALF : 0) + (PA_KV - 1 - (c >> 4)) * 128)[c & 7] = make_uint4(0u, 0u, 0u, 0u);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // before the products read them
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(&t->v_clean)) : "memory");
+            }
+        }
     } else if (warp == 1) {
         if (lane == 0 && n_tiles > 0) {
             // D f32, A and B bf16, N = 128 (OW), M = 128; the second product's B is MN-major
@@ -385,7 +399,7 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
                 }
                 umma_commit(&t->k_empty);
                 umma_commit(&t->s_full);
-                ok = wait(&t->v_full, i & 1, 2u) && wait(&t->p_full, i & 1, 2u);
+                ok = wait(&t->v_full, i & 1, 2u) && (stale == 0 || i + 1 < n_tiles || wait(&t->v_clean, 0, 2u)) && wait(&t->p_full, i & 1, 2u);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t dv = desc_mn_sw128(vs);
@@ -407,26 +421,6 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
         float m_run = -INFINITY, l_run = 0.f;            // maximum in log2 units
         bool ok = true;
         for (int i = 0; i < n_tiles; ++i) {
-            if ((i + 1) * PA_KV - 1 > first + m0) {      // V rows of this tile that some query must not see (uniform over the CTA)
-                ok = wait(&t->v_full, i & 1, 3u);
-                if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-                const int pos = i * PA_KV + r;           // this thread's V row; its 16-byte pieces in the order that meets no bank twice
-                uint4* row = reinterpret_cast<uint4*>(vs + r * 128);
-                uint32_t most = 0;                       // the largest magnitudes of even and odd elements
-#pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    uint4* piece = row + (c >> 3) * (PA_HALF / 16) + ((c + r) & 7);
-                    if (pos > last) {
-                        *piece = make_uint4(0u, 0u, 0u, 0u);
-                    } else if (!MLA || c < 8) {          // (latent form: a value's first term tells)
-                        const uint4 u = *piece;
-                        most = __vmaxu2(__vmaxu2(__vmaxu2(most, u.x & 0x7fff7fffu), __vmaxu2(u.y & 0x7fff7fffu, u.z & 0x7fff7fffu)),
-                                        u.w & 0x7fff7fffu);
-                    }
-                }
-                if (pos > first + m0 && ((most & 0xffffu) >= 0x7f80u || (most >> 16) >= 0x7f80u)) t->poisoned = 1;
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the zeros, before the products read them
-            }
             ok = wait(&t->s_full, i & 1, 3u);
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -501,18 +495,19 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(&t->p_full)) : "memory");
         }
         if (ok) ok = wait(&t->o_done, (n_tiles - 1) & 1, 3u);
-        asm volatile("bar.sync 1, 128;" ::: "memory");   // every warp has looked at its V rows
-        if (t->poisoned) {
-            slow_rows<G, MLA>(p, first, m0, g, quad * 32, lane);
-        } else if (__all_sync(0xffffffffu, ok)) {
+        if (__all_sync(0xffffffffu, ok)) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const float inv = 1.f / l_run;
             uint16_t* dst = p.out + (size_t(tok) * p.hq + g * G + r % G) * OW;
+            const bool mine = tok < p.m && my_pos < p.max_ctx;
+            uint32_t most = __float_as_uint(inv) & 0x7fffffffu;          // the largest magnitude: not finite?
 #pragma unroll 1
             for (int c = 0; c < OW; c += 32) {
                 uint32_t v[32];
                 tmem_ld32(v, trow + 128 + c);
-                if (tok < p.m && my_pos < p.max_ctx) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) most = max(most, v[j] & 0x7fffffffu);
+                if (mine) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         uint4 w;
@@ -523,6 +518,10 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
                         *reinterpret_cast<uint4*>(dst + c + 8 * q) = w;
                     }
                 }
+            }
+            if (__any_sync(0xffffffffu, mine && most >= 0x7f800000u)) {
+                __syncwarp();                            // (these results are written over)
+                slow_rows<G, MLA>(p, first, m0, g, quad * 32, lane);
             }
         }
     }
