@@ -39,6 +39,10 @@ enum {
     TFB_ENODEVICE = 5    /* no sm_100 device is current */
 };
 
+/* Grows with every change of an argument structure: a caller compares what it was built against with tfb_version() before
+ * its first call (a structure that a caller knows shorter would be read past its end).  101: n_prompt_at at the end of the
+ * head's, the steps' and the nucleus draw's structures; the wide form of tfb_minicpm3_prefill_args. */
+#define TFB_VERSION 101
 TFB_API int tfb_version(void);
 TFB_API const char* tfb_status_string(int status);
 /* Text of the last CUDA runtime error a launch returned on this thread ("" if none). */

@@ -271,3 +271,13 @@ def test_qwen35_chunks_refuse_shapes_and_layers_their_kernels_do_not_hold(so):
         for n in names + ("gamma_in", "w_in", "w_out", "gamma_post", "w_router", "w_gate", "w_up", "w_down", "w_shared_gate"):
             assert call({"kind": kind, n: None}) == EINVAL, (kind, n)
     assert call({"gamma_gdn": ODD}) == EALIGN and call({"kind": 1, "k_pool": ODD}) == EALIGN and call({"w_in": ODD}) == EALIGN
+
+
+def test_header_library_and_binding_are_of_one_version(so, monkeypatch):
+    import re
+    from pathlib import Path
+    header = (Path(lib.__file__).resolve().parents[1] / "include" / "tfb200.h").read_text()
+    assert int(re.search(r"#define TFB_VERSION (\d+)", header).group(1)) == so.tfb_version() == lib.VERSION
+    monkeypatch.setattr(lib, "VERSION", lib.VERSION + 1)
+    with pytest.raises(RuntimeError, match="rebuild"):
+        getattr(lib.load, "__wrapped__", lib.load)()

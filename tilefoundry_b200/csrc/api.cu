@@ -31,7 +31,7 @@ using namespace tfb::host;
 
 extern "C" {
 
-int tfb_version(void) { return 100; }
+int tfb_version(void) { return TFB_VERSION; }
 
 int tfb_debug_trace(void* device_buffer, int32_t capacity) {
     g_trace_buf = static_cast<unsigned long long*>(device_buffer);

@@ -228,6 +228,9 @@ class GraniteStepArgs(C.Structure):
                 ("eos_ids", _vp), ("stop_at", _vp), ("n_eos", _i32), ("reserved_eos", _i32), ("n_prompt_at", _vp)]
 
 
+#: ``TFB_VERSION`` of the header these structures mirror
+VERSION = 101
+
 #: every symbol ``include/tfb200.h`` declares: name -> (restype, argtypes)
 class GemvF32Args(C.Structure):
     _fields_ = [("w", _vp), ("w2", _vp), ("w_extra", _vp), ("w2_extra", _vp), ("x", _vp), ("gamma", _vp), ("gate", _vp),
@@ -375,6 +378,9 @@ def load() -> C.CDLL:
     for name, (res, args) in SYMBOLS.items():
         fn = getattr(lib, name)
         fn.restype, fn.argtypes = res, args
+    if lib.tfb_version() != VERSION:
+        raise RuntimeError(f"{LIB_PATH} is version {lib.tfb_version()}, this binding is {VERSION}: rebuild it with "
+                           "`python -m tilefoundry_b200.build --force`")
     return lib
 
 
