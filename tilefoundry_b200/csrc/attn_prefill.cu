@@ -43,7 +43,7 @@ constexpr int PA_TILE = 2 * PA_HALF;
 constexpr float kLog2e = 1.4426950408889634f;
 
 struct PaTail {
-    uint64_t q_full, k_full, v_full, v_clean, k_empty, v_empty, s_full, p_full, o_done;
+    uint64_t q_full, k_full, v_full, v_clean, k_empty, v_empty, s_full, p_full, o_done, drain;
     uint32_t tmem_base;
     volatile int aborted;
 };
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
     if (threadIdx.x == 0) {
         mbar_init(&t->q_full, 1); mbar_init(&t->k_full, 1); mbar_init(&t->v_full, 1); mbar_init(&t->v_clean, 1);
         mbar_init(&t->k_empty, 1); mbar_init(&t->v_empty, 1); mbar_init(&t->s_full, 1);
-        mbar_init(&t->p_full, 4); mbar_init(&t->o_done, 1);
+        mbar_init(&t->p_full, 4); mbar_init(&t->o_done, 1); mbar_init(&t->drain, 1);
         t->aborted = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
         atomicExch(p.status, role);
         return false;
     };
+    int asked = 0;                                       // (the producer's K and V tiles: 2 i + 1 after K of tile i, 2 i + 2 after its V)
 
     if (warp == 0) {
         if (lane == 0 && n_tiles > 0) {
@@ -356,9 +357,11 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
                 ok = wait(&t->k_empty, (i & 1) ^ 1, 1u);
                 if (!ok) break;
                 if (MLA) load_mla(ks, &t->k_full, i, true); else load(ks, &map_k, &t->k_full, i);
+                asked = 2 * i + 1;
                 ok = wait(&t->v_empty, (i & 1) ^ 1, 1u);
                 if (!ok) break;
                 if (MLA) load_mla(vs, &t->v_full, i, false); else load(vs, &map_v, &t->v_full, i);
+                asked = 2 * i + 2;
             }
         }
         __syncwarp();
@@ -528,6 +531,15 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (t->aborted) {                                    // what is in flight ends (bounded) before its memory is given back
+        if (threadIdx.x == 0) {
+            if (n_tiles > 0) mbar_wait(&t->q_full, 0);
+            if (asked > 0) mbar_wait(&t->k_full, ((asked + 1) / 2 - 1) & 1);
+            if (asked > 1) mbar_wait(&t->v_full, (asked / 2 - 1) & 1);
+        }
+        if (warp == 1 && lane == 0) drain_products(&t->drain);
+        __syncthreads();
+    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(256u) : "memory");

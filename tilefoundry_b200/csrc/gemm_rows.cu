@@ -32,7 +32,7 @@ constexpr int RW_A_TILE = RW_BM * RW_BK * 2, RW_A_BYTES = RW_KB * RW_A_TILE;
 constexpr int RW_BN = 128, RW_B_TILE = RW_BN * RW_BK * 2, RW_B_BYTES = RW_KB * RW_B_TILE, RW_STAGES = 3;
 
 struct RwSmemTail {
-    uint64_t full[RW_STAGES], empty[RW_STAGES], acc_full[2], acc_empty[2];
+    uint64_t full[RW_STAGES], empty[RW_STAGES], acc_full[2], acc_empty[2], drain;
     uint32_t tmem_base;
     volatile int aborted;
 };
@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_rows_kernel(const __grid_c
     if (threadIdx.x == 0) {
         for (int s = 0; s < ST; ++s) { mbar_init(&t->full[s], 1); mbar_init(&t->empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&t->acc_full[b], 1); mbar_init(&t->acc_empty[b], 4); }
+        mbar_init(&t->drain, 1);
         t->aborted = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_rows_kernel(const __grid_c
         atomicExch(p.status, role);
         return false;
     };
+    int issued = 0;                                                     // (the producer's K steps)
 
     if (warp == 0) {
         if (lane == 0) {                                                // ---- TMA producer ----
@@ -184,6 +186,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_rows_kernel(const __grid_c
             }
             pdl_wait();
             for (int k = 0; k < pre; ++k) load_x(blockIdx.x, k, k);
+            issued = pre;
             s = pre == ST ? 0 : pre;
             ph = pre == ST ? 1u : 0u;
             bool ok = true;
@@ -194,6 +197,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_rows_kernel(const __grid_c
                     mbar_expect_tx(&t->full[s], RW_A_BYTES + BB);
                     load_w(tile, k, s);
                     load_x(tile, k, s);
+                    ++issued;
                     if (++s == ST) { s = 0; ph ^= 1u; }
                 }
             }
@@ -245,6 +249,11 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_rows_kernel(const __grid_c
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (t->aborted) {
+        if (threadIdx.x == 0) drain_copies(t->full, issued);
+        if (warp == 1 && lane == 0) drain_products(&t->drain);
+        __syncthreads();
+    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(uint32_t(2 * BN)) : "memory");
@@ -290,7 +299,7 @@ cudaError_t launch_rows(const void* w, const void* x, TcParams p, cudaStream_t s
 constexpr int PR_BN = 256, PR_TILE = 128 * RW_BK * 2, PR_HALF = RW_KB * PR_TILE, PR_STAGES = 3;
 
 struct PrSmemTail {
-    uint64_t full[PR_STAGES], empty[PR_STAGES], acc_full[2], acc_empty[2];
+    uint64_t full[PR_STAGES], empty[PR_STAGES], acc_full[2], acc_empty[2], drain;
     uint32_t tmem_base;
     volatile int aborted;
 };
@@ -334,6 +343,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_pair_kernel(const __grid_c
     if (threadIdx.x == 0) {
         for (int s = 0; s < PR_STAGES; ++s) { mbar_init(&t->full[s], 1); mbar_init(&t->empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&t->acc_full[b], 1); mbar_init(&t->acc_empty[b], 8); }
+        mbar_init(&t->drain, 1);
         t->aborted = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -356,6 +366,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_pair_kernel(const __grid_c
         atomicExch(p.status, role);
         return false;
     };
+    int issued = 0;                                                     // (the producer's K steps)
 
     if (warp == 0) {
         if (lane == 0) {                                                // ---- TMA producer: one in each CTA ----
@@ -376,6 +387,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_pair_kernel(const __grid_c
             }
             pdl_wait();
             for (int k = 0; k < pre; ++k) load_x(first, k, k);
+            issued = pre;
             int s = pre == PR_STAGES ? 0 : pre;
             uint32_t ph = pre == PR_STAGES ? 1u : 0u;
             bool ok = true;
@@ -386,6 +398,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_pair_kernel(const __grid_c
                     expect(s);
                     load_w(tile, k, s);
                     load_x(tile, k, s);
+                    ++issued;
                     if (++s == PR_STAGES) { s = 0; ph ^= 1u; }
                 }
         }
@@ -438,6 +451,13 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_pair_kernel(const __grid_c
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (t->aborted && rank == 0) {                                      // (its barriers count the copies of both CTAs, its thread issued the products)
+        if (threadIdx.x == 0) drain_copies(t->full, issued);
+        if (warp == 1 && lane == 0) {
+            asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&t->drain)) : "memory");
+            mbar_wait(&t->drain, 0);
+        }
+    }
     cluster_sync();                                                     // nobody leaves while the pair's products or barriers need it
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

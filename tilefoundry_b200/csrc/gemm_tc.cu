@@ -53,7 +53,7 @@ template <int BN> struct TcShape {
 
 template <int BN>
 struct TcSmemTail {
-    uint64_t full[TcShape<BN>::kStages], empty[TcShape<BN>::kStages], accum;
+    uint64_t full[TcShape<BN>::kStages], empty[TcShape<BN>::kStages], accum, drain;
     uint32_t tmem_base;
     int aborted;
 };
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcShape<BN>::kCtas) gemm_tc_kernel
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < ST; ++s) { mbar_init(&t->full[s], 1); mbar_init(&t->empty[s], 1); }
-        mbar_init(&t->accum, 1);
+        mbar_init(&t->accum, 1); mbar_init(&t->drain, 1);
         t->aborted = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcShape<BN>::kCtas) gemm_tc_kernel
     pdl_trigger();
     const bool producer = (warp == 0 && lane == 0);
     if (!producer) pdl_wait();
+    int issued = 0;                                                     // (the producer's)
 
     if (warp == 0) {
         if (lane == 0) {                                                // ---- TMA producer ----
@@ -217,12 +218,14 @@ __global__ void __launch_bounds__(TC_THREADS, TcShape<BN>::kCtas) gemm_tc_kernel
             }
             pdl_wait();
             for (int i = 0; i < pre; ++i) tma_load_2d(stage(i) + TC_A_BYTES, &map_x, &t->full[i], (k_begin + i) * TC_BK, m0);
+            issued = pre;
             for (int i = pre; i < nsteps; ++i) {
                 const int s = i % ST;
                 if (!mbar_wait(&t->empty[s], ((i / ST) & 1) ^ 1)) { t->aborted = 1; atomicExch(p.status, 1u); break; }
                 mbar_expect_tx(&t->full[s], STAGE);
                 tma_load_w(stage(s), &map_w, &t->full[s], (k_begin + i) * TC_BK, row);
                 tma_load_2d(stage(s) + TC_A_BYTES, &map_x, &t->full[s], (k_begin + i) * TC_BK, m0);
+                issued = i + 1;
             }
         }
     } else if (warp == 1) {
@@ -265,6 +268,11 @@ __global__ void __launch_bounds__(TC_THREADS, TcShape<BN>::kCtas) gemm_tc_kernel
     // ---- teardown, and the split-K reduction through distributed shared memory ----
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (t->aborted) {
+        if (producer) drain_copies(t->full, issued);
+        if (warp == 1 && lane == 0) drain_products(&t->drain);
+        __syncthreads();
+    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(uint32_t(BN)) : "memory");

@@ -48,6 +48,18 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(bar)) : "memory");
 }
 
+// After a wait of this CTA gave up (all roles are past their loops): the `issued` newest uses of a ring's stages, bounded waits
+// as all others, so that no copy lands in memory that has been given back.  By the thread that asked for the copies.
+template <int STAGES>
+__device__ __forceinline__ void drain_copies(uint64_t (&full)[STAGES], int issued) {
+    for (int i = max(issued - STAGES, 0); i < issued; ++i) mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
+}
+// ... and the products, by the thread that issued them, before their tensor memory is given back.
+__device__ __forceinline__ void drain_products(uint64_t* bar) {
+    umma_commit(bar);
+    mbar_wait(bar, 0);
+}
+
 // 32 columns of this warp's tensor-memory lane quadrant, one row per lane; the registers are valid after tmem_wait_ld
 __device__ __forceinline__ void tmem_ld32_async(uint32_t (&v)[32], uint32_t taddr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
