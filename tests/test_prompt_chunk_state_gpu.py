@@ -53,8 +53,8 @@ def test_chunks_leave_both_convolution_windows(qwen35, pieces):
 
 @pytest.mark.parametrize("use_graph", [False, True])
 def test_steps_inside_a_prompt_leave_their_logits_and_picks(qwen35, use_graph):
-    """``run`` takes every position as a step, also at the start of a sequence: a caller who scores a prompt piece by piece
-    reads each piece's last logits and pick, and nothing waits for the device."""
+    """``run`` takes the positions of a part of a prompt as steps: a caller who scores a prompt piece by piece reads each
+    piece's last logits and pick, and nothing waits for the device."""
     (walk, prompt), (sess, _) = qwen35(10), qwen35(10)
     walk.reset(prompt)
     sess.generate(prompt.flip(0), 1)                     # another request's logits and pick lie there
@@ -70,6 +70,25 @@ def test_steps_inside_a_prompt_leave_their_logits_and_picks(qwen35, use_graph):
         assert torch.equal(sess.logits, walk.logits) and int(sess.picked) == int(walk.picked) and int(sess.pos) == int(walk.pos)
     for got, want in zip(sess.state_tensors(), walk.state_tensors()):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("steps", [10, 11, 25])
+def test_steps_past_a_prompt_go_on_as_generate_does(qwen35, steps):
+    (gen, prompt), (sess, _) = qwen35(10), qwen35(10)
+    want = gen.generate(prompt, steps - 9).tokens
+    sess.reset(prompt)
+    start = sess.snapshot()
+    for _ in range(2):                                   # (and again from the start)
+        sess.run(steps)
+        assert sess.tokens[10: steps + 1].tolist() == want and int(sess.pos) == steps and int(sess.picked) == want[-1]
+        assert torch.equal(sess.logits, gen.logits)
+        for got, other in zip(sess.state_tensors(), gen.state_tensors()):
+            assert torch.equal(got, other)
+        sess.restore(start)
+    sess.run(4)                                          # not at the start any more: no chunk may begin there
+    sess.run(12)
+    sess.check_prompt()
+    assert int(sess.pos) == 16
 
 
 def _chunked_session(model, qwen35):

@@ -210,6 +210,7 @@ class Qwen35Session(DecodeSession):
         for layer in self._recurrent():               # recurrent state starts at zero for a new sequence
             layer["conv_state"].zero_()
             layer["state"].zero_()
+        self._at_start = True
 
     def state_tensors(self) -> list:
         return [l[n] for l in self._recurrent() for n in ("conv_state", "state")]
@@ -255,6 +256,28 @@ class Qwen35Session(DecodeSession):
         if not self._chunked():
             raise ValueError("chunked prompt processing is not built for this session")
         self._chunks().run(n_tokens, first)
+
+    _at_start = False                                # perhaps: since a ``reset`` or ``restore`` nobody has looked
+
+    def restore(self, snap: dict) -> None:
+        super().restore(snap)
+        self._at_start = True
+
+    def run(self, steps: int, use_graph: bool = True) -> None:
+        """As DecodeSession.run.  Where the sequence stands at its start and the *steps* reach past its prompt, the prompt goes
+        through as in ``generate`` (the same tokens follow); a part of a prompt is taken step by step, each step leaving its
+        logits and pick.  The one device read of it: where the sequence stands, once after a ``reset`` or ``restore``."""
+        if (self._at_start and steps >= self.n_prompt >= 3 and self.trace is None and self._chunked()
+                and not torch.cuda.is_current_stream_capturing()):
+            self._at_start = False
+            if int(self.pos.item()) == 0:
+                if use_graph and self.graph is None:
+                    self.capture()                       # (ahead of the prompt: its warm-up steps leave logits and picks)
+                last = self._chunks().run(self.n_prompt, 0, pick=True)
+                if last is not None:
+                    self._pick_from(last)
+                steps -= self.n_prompt
+        super().run(steps, use_graph)
 
     def generate(self, prompt_ids, max_new: int, use_graph: bool = True, eos=None, *, prefill: bool = True):
         """As DecodeSession.generate.  The prompt goes through in chunks where the session has them and a token is picked
