@@ -19,8 +19,8 @@
 // next 16 their lo terms.  O is only rescaled when a row's maximum has grown by more than 8 (in log2), exact either way.
 //
 // The product meets every row of a V tile, so a row that a query must not see is more than a weight of zero (0 x Inf and
-// 0 x NaN are NaN).  Rows past the chunk (a page's stale rows) are zeroed in shared memory by the requesting warp
-// while the softmax runs (by the softmax warps themselves it cost 1.5 us a layer); a warp one of whose
+// 0 x NaN are NaN).  Rows past the chunk (a page's stale rows) are zeroed in shared memory by the requesting
+// warp while the softmax runs (by the softmax warps themselves it cost 1.5 us a layer); a warp one of whose
 // results is not finite -- a later token of the tile may have done that, or an earlier one rightly -- takes its
 // rows again by a plain walk over the positions each query sees (slow_rows), as the decode kernels take them.  (Looking through
 // the V tile for such values instead cost 1.6 us a layer.)
@@ -89,6 +89,12 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     uint32_t r;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// c + 0 * a of bf16 pairs: NaN where a is not finite
+__device__ __forceinline__ uint32_t times_zero(uint32_t a, uint32_t c) {
+    uint32_t r;
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(0u), "r"(c));
     return r;
 }
 __device__ __forceinline__ float ex2(float x) {
@@ -324,7 +330,6 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
         atomicExch(p.status, role);
         return false;
     };
-    int asked = 0;                                       // (the producer's K and V tiles: 2 i + 1 after K of tile i, 2 i + 2 after its V)
 
     if (warp == 0) {
         if (lane == 0 && n_tiles > 0) {
@@ -353,15 +358,21 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
                     for (int q = 0; q < 2; ++q) tma_load_3d(dst + PA_TILE + q * (PA_HALF / 4), &map_kr, bar, 256, 0, page_row(tile, q));
             };
             bool ok = true;
+            int n_k = 0, n_v = 0;
             for (int i = 0; i < n_tiles && ok; ++i) {
                 ok = wait(&t->k_empty, (i & 1) ^ 1, 1u);
                 if (!ok) break;
                 if (MLA) load_mla(ks, &t->k_full, i, true); else load(ks, &map_k, &t->k_full, i);
-                asked = 2 * i + 1;
+                n_k = i + 1;
                 ok = wait(&t->v_empty, (i & 1) ^ 1, 1u);
                 if (!ok) break;
                 if (MLA) load_mla(vs, &t->v_full, i, false); else load(vs, &map_v, &t->v_full, i);
-                asked = 2 * i + 2;
+                n_v = i + 1;
+            }
+            if (!ok) {
+                drain_copies(&t->q_full, 1, 1);
+                drain_copies(&t->k_full, 1, n_k);
+                drain_copies(&t->v_full, 1, n_v);
             }
         }
         __syncwarp();
@@ -416,6 +427,7 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
                 umma_commit(&t->v_empty);
                 umma_commit(&t->o_done);
             }
+            if (!ok) drain_products(&t->drain);
         }
     } else if (n_tiles > 0) {
         const int quad = warp & 3, r = quad * 32 + lane; // query row: token r / G of the tile, head r % G
@@ -503,13 +515,11 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
             const float inv = 1.f / l_run;
             uint16_t* dst = p.out + (size_t(tok) * p.hq + g * G + r % G) * OW;
             const bool mine = tok < p.m && my_pos < p.max_ctx;
-            uint32_t most = __float_as_uint(inv) & 0x7fffffffu;          // the largest magnitude: not finite?
+            uint32_t odd = 0;                            // two bf16 zeros as long as every result is finite
 #pragma unroll 1
             for (int c = 0; c < OW; c += 32) {
                 uint32_t v[32];
                 tmem_ld32(v, trow + 128 + c);
-#pragma unroll
-                for (int j = 0; j < 32; ++j) most = max(most, v[j] & 0x7fffffffu);
                 if (mine) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
@@ -519,10 +529,11 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
                         w.z = pack2(__uint_as_float(v[8 * q + 4]) * inv, __uint_as_float(v[8 * q + 5]) * inv);
                         w.w = pack2(__uint_as_float(v[8 * q + 6]) * inv, __uint_as_float(v[8 * q + 7]) * inv);
                         *reinterpret_cast<uint4*>(dst + c + 8 * q) = w;
+                        odd = times_zero(w.x, times_zero(w.y, times_zero(w.z, times_zero(w.w, odd))));
                     }
                 }
             }
-            if (__any_sync(0xffffffffu, mine && most >= 0x7f800000u)) {
+            if (__any_sync(0xffffffffu, (odd & 0x7fff7fffu) != 0u)) {
                 __syncwarp();                            // (these results are written over)
                 slow_rows<G, MLA>(p, first, m0, g, quad * 32, lane);
             }
@@ -531,15 +542,6 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (t->aborted) {                                    // what is in flight ends (bounded) before its memory is given back
-        if (threadIdx.x == 0) {
-            if (n_tiles > 0) mbar_wait(&t->q_full, 0);
-            if (asked > 0) mbar_wait(&t->k_full, ((asked + 1) / 2 - 1) & 1);
-            if (asked > 1) mbar_wait(&t->v_full, (asked / 2 - 1) & 1);
-        }
-        if (warp == 1 && lane == 0) drain_products(&t->drain);
-        __syncthreads();
-    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(256u) : "memory");

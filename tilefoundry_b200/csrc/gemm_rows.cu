@@ -166,7 +166,6 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_rows_kernel(const __grid_c
         atomicExch(p.status, role);
         return false;
     };
-    int issued = 0;                                                     // (the producer's K steps)
 
     if (warp == 0) {
         if (lane == 0) {                                                // ---- TMA producer ----
@@ -186,7 +185,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_rows_kernel(const __grid_c
             }
             pdl_wait();
             for (int k = 0; k < pre; ++k) load_x(blockIdx.x, k, k);
-            issued = pre;
+            int issued = pre;
             s = pre == ST ? 0 : pre;
             ph = pre == ST ? 1u : 0u;
             bool ok = true;
@@ -201,6 +200,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_rows_kernel(const __grid_c
                     if (++s == ST) { s = 0; ph ^= 1u; }
                 }
             }
+            if (!ok) drain_copies(t->full, ST, issued);
         }
     } else if (warp == 1) {
         if (lane == 0) {                                                // ---- MMA issuer ----
@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_rows_kernel(const __grid_c
                 if (ok) umma_commit(&t->acc_full[buf]);
                 if (++buf == 2) { buf = 0; aph ^= 1u; }
             }
+            if (!ok) drain_products(&t->drain);
         }
     } else {                                                            // ---- epilogue: warps 2..5 ----
         const int quad = warp & 3;                                      // the tensor-memory lane quadrant this warp may read
@@ -249,11 +250,6 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_rows_kernel(const __grid_c
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (t->aborted) {
-        if (threadIdx.x == 0) drain_copies(t->full, issued);
-        if (warp == 1 && lane == 0) drain_products(&t->drain);
-        __syncthreads();
-    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(uint32_t(2 * BN)) : "memory");
@@ -366,7 +362,6 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_pair_kernel(const __grid_c
         atomicExch(p.status, role);
         return false;
     };
-    int issued = 0;                                                     // (the producer's K steps)
 
     if (warp == 0) {
         if (lane == 0) {                                                // ---- TMA producer: one in each CTA ----
@@ -387,7 +382,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_pair_kernel(const __grid_c
             }
             pdl_wait();
             for (int k = 0; k < pre; ++k) load_x(first, k, k);
-            issued = pre;
+            int issued = pre;
             int s = pre == PR_STAGES ? 0 : pre;
             uint32_t ph = pre == PR_STAGES ? 1u : 0u;
             bool ok = true;
@@ -401,6 +396,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_pair_kernel(const __grid_c
                     ++issued;
                     if (++s == PR_STAGES) { s = 0; ph ^= 1u; }
                 }
+            if (!ok && rank == 0) drain_copies(t->full, PR_STAGES, issued);      // (its barriers count the copies of both CTAs)
         }
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {                                   // ---- MMA issuer of the pair ----
@@ -429,6 +425,10 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_pair_kernel(const __grid_c
                 if (ok) umma_commit_pair(&t->acc_full[buf]);
                 if (++buf == 2) { buf = 0; aph ^= 1u; }
             }
+            if (!ok) {
+                asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&t->drain)) : "memory");
+                mbar_wait(&t->drain, 0);
+            }
         }
     } else {                                                            // ---- epilogue: warps 2..5 of both CTAs ----
         const int quad = warp & 3;
@@ -451,13 +451,6 @@ __global__ void __launch_bounds__(RW_THREADS, 1) gemm_pair_kernel(const __grid_c
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (t->aborted && rank == 0) {                                      // (its barriers count the copies of both CTAs, its thread issued the products)
-        if (threadIdx.x == 0) drain_copies(t->full, issued);
-        if (warp == 1 && lane == 0) {
-            asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&t->drain)) : "memory");
-            mbar_wait(&t->drain, 0);
-        }
-    }
     cluster_sync();                                                     // nobody leaves while the pair's products or barriers need it
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -205,7 +205,6 @@ __global__ void __launch_bounds__(TC_THREADS, TcShape<BN>::kCtas) gemm_tc_kernel
     pdl_trigger();
     const bool producer = (warp == 0 && lane == 0);
     if (!producer) pdl_wait();
-    int issued = 0;                                                     // (the producer's)
 
     if (warp == 0) {
         if (lane == 0) {                                                // ---- TMA producer ----
@@ -218,14 +217,17 @@ __global__ void __launch_bounds__(TC_THREADS, TcShape<BN>::kCtas) gemm_tc_kernel
             }
             pdl_wait();
             for (int i = 0; i < pre; ++i) tma_load_2d(stage(i) + TC_A_BYTES, &map_x, &t->full[i], (k_begin + i) * TC_BK, m0);
-            issued = pre;
             for (int i = pre; i < nsteps; ++i) {
                 const int s = i % ST;
-                if (!mbar_wait(&t->empty[s], ((i / ST) & 1) ^ 1)) { t->aborted = 1; atomicExch(p.status, 1u); break; }
+                if (!mbar_wait(&t->empty[s], ((i / ST) & 1) ^ 1)) {
+                    t->aborted = 1;
+                    atomicExch(p.status, 1u);
+                    drain_copies(t->full, ST, i);
+                    break;
+                }
                 mbar_expect_tx(&t->full[s], STAGE);
                 tma_load_w(stage(s), &map_w, &t->full[s], (k_begin + i) * TC_BK, row);
                 tma_load_2d(stage(s) + TC_A_BYTES, &map_x, &t->full[s], (k_begin + i) * TC_BK, m0);
-                issued = i + 1;
             }
         }
     } else if (warp == 1) {
@@ -245,6 +247,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcShape<BN>::kCtas) gemm_tc_kernel
                 umma_commit(&t->empty[s]);                              // arrives when these MMAs have read the stage
             }
             if (ok) umma_commit(&t->accum);                             // arrives when the accumulator is complete
+            else drain_products(&t->drain);
         }
     } else {                                                            // ---- warps 2..5 read the accumulator back ----
         const int quad = warp & 3;                                      // the TMEM lane quadrant this warp may read
@@ -268,11 +271,6 @@ __global__ void __launch_bounds__(TC_THREADS, TcShape<BN>::kCtas) gemm_tc_kernel
     // ---- teardown, and the split-K reduction through distributed shared memory ----
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (t->aborted) {
-        if (producer) drain_copies(t->full, issued);
-        if (warp == 1 && lane == 0) drain_products(&t->drain);
-        __syncthreads();
-    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(uint32_t(BN)) : "memory");

@@ -48,14 +48,14 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(bar)) : "memory");
 }
 
-// After a wait of this CTA gave up (all roles are past their loops): the `issued` newest uses of a ring's stages, bounded waits
-// as all others, so that no copy lands in memory that has been given back.  By the thread that asked for the copies.
-template <int STAGES>
-__device__ __forceinline__ void drain_copies(uint64_t (&full)[STAGES], int issued) {
-    for (int i = max(issued - STAGES, 0); i < issued; ++i) mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
+// A role that leaves its loop because a wait gave up: the `issued` newest uses of a ring's stages, bounded waits as all others,
+// so that no copy lands in memory that has been given back.  (A role that has finished by then leaves nothing in flight: the
+// wait that gave up was a million polls long.)  Calls, not inlined: a launch fetches every line of code it passes over.
+static __device__ __noinline__ void drain_copies(uint64_t* full, int stages, int issued) {
+    for (int i = max(issued - stages, 0); i < issued; ++i) mbar_wait(full + i % stages, (i / stages) & 1);
 }
-// ... and the products, by the thread that issued them, before their tensor memory is given back.
-__device__ __forceinline__ void drain_products(uint64_t* bar) {
+// ... and the products, by the thread that issued them.
+static __device__ __noinline__ void drain_products(uint64_t* bar) {
     umma_commit(bar);
     mbar_wait(bar, 0);
 }
