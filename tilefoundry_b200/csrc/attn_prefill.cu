@@ -433,7 +433,9 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
         const int quad = warp & 3, r = quad * 32 + lane; // query row: token r / G of the tile, head r % G
         const uint32_t trow = tmem + (uint32_t(quad * 32) << 16);
         const int tok = m0 + r / G, my_pos = first + tok;
-        float m_run = -INFINITY, l_run = 0.f;            // maximum in log2 units
+        // maximum in log2 units: below any score worth a weight, but a number (a row all of whose scores are -infinity or
+        // lower than this gets no weight, and with it the plain walk)
+        float m_run = -1e30f, l_run = 0.f;
         bool ok = true;
         for (int i = 0; i < n_tiles; ++i) {
             ok = wait(&t->s_full, i & 1, 3u);
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
             float mx = fmaxf(fmaxf(mq[0], mq[1]), fmaxf(mq[2], mq[3]));
             mx *= kLog2e;
             // keep the reference maximum until a row outgrows it by 2^8 (always exact: it divides out)
-            const bool grow = mx > m_run + 8.f || (m_run == -INFINITY && mx > -INFINITY);
+            const bool grow = mx > m_run + 8.f;
             if (i > 0) {                                 // O holds the last tile's products before anything touches it
                 ok = wait(&t->o_done, (i - 1) & 1, 3u);
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
@@ -471,8 +473,7 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
             }
             if (__any_sync(0xffffffffu, grow)) {
                 const float m_new = grow ? mx : m_run;
-                const float f = m_run == -INFINITY ? 0.f : ex2(m_run - m_new);
-                const float scale = grow ? f : 1.f;
+                const float scale = grow ? ex2(m_run - m_new) : 1.f;
                 if (i > 0) {
 #pragma unroll 1
                     for (int c = 0; c < OW; c += 32) {
@@ -486,15 +487,14 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prefill_attn_kernel(const __gri
                 l_run *= scale;
                 m_run = m_new;
             }
-            const float m_ref = m_run == -INFINITY ? 0.f : m_run;        // (no score above -infinity yet: no weight)
 #pragma unroll
             for (int c = 0; c < PA_KV / 32; ++c) {
                 uint32_t o[32];
                 float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
                 for (int j = 0; j < 32; j += 2) {
-                    const float a = ex2(fmaf(__uint_as_float(v[c][j]), kLog2e, -m_ref));
-                    const float b = ex2(fmaf(__uint_as_float(v[c][j + 1]), kLog2e, -m_ref));
+                    const float a = ex2(fmaf(__uint_as_float(v[c][j]), kLog2e, -m_run));
+                    const float b = ex2(fmaf(__uint_as_float(v[c][j + 1]), kLog2e, -m_run));
                     sum0 += a;
                     sum1 += b;
                     const uint32_t hi = pack2(a, b);
