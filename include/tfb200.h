@@ -819,10 +819,11 @@ typedef struct {
     uint32_t* status;
     int32_t tokens, hidden, inter, experts, top_k, pdl;
 } tfb_moe_batch_args;
+/* An index outside 0 .. experts-1 is on no list (that slot of y keeps what it held). */
 TFB_API int tfb_moe_batch(const tfb_moe_batch_args* args, tfb_stream_t stream);
 /* Routing for the same batch: logits[t][e] = bf16(W_router[e] . bf16 x[t]) (row `experts`: the shared expert's scale row),
  * then the selection of tfb_router_select (mode 0: top-k then softmax over the k; mode 1: softmax over all, top-k,
- * renormalise) for every token, one CTA per token.  `routing` + the gate logit of `shared_expert` of the authored
+ * renormalise) for every token, a warp per token: top_k different experts whatever the logits.  `routing` + the gate logit of `shared_expert` of the authored
  * block for a batch (examples/qwen3_5_35b_a3b-tilelang/model.py: routing, shared_expert); weights are f32.
  * hidden a multiple of 256 up to 8192, experts <= 256, top_k <= 32. */
 typedef struct {
@@ -898,7 +899,8 @@ TFB_API int tfb_qwen3_batch_decode_step(const tfb_qwen3_batch_step_args* args, t
  * attention on the tensor cores where the head width is 128, a page holds a multiple of 64 positions and 1, 2 or 4
  * query heads share a KV head, else in the chunk form of tfb_attn_gqa_decode (every token attends to the cached rows
  * before it; see `chunk` there; part_o, part_ml and counters are only used then).  m is at most
- * tfb_qwen3_prefill_max_chunk of the shapes: 4096 with the flash form, else 32.  Two launches per layer either way.  Leaves the tokens' K/V rows in the cache and the residual stream of
+ * tfb_qwen3_prefill_max_chunk of the shapes: 4096 with the flash form, else 32.  Two launches of a layer are its attention's
+ * either way.  Cache rows past the chunk and rows that a token does not see are never multiplied.  Leaves the tokens' K/V rows in the cache and the residual stream of
  * each token in hidden_buf; no head, no pick: a prompt's logits are not needed until its last token, which the
  * decode step processes.  The reference walks a prompt token by token
  * (tests/models/orchestrator/causal_lm/generation.py:56-61); per token the arithmetic and its rounding points are
