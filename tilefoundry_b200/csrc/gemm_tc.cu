@@ -290,11 +290,12 @@ static int splits_for_tiles(int tiles, int k, int resident, int most) {
 // Up to 128 tokens two CTAs share an SM, worth it up to 4 splits (6400 gate/up pairs x 2560, 128 tokens: two splits 20.1 us,
 // unsplit 23.8; 8192 x 2048: four 13.5, two 15.9; the MiniCPM3 prompt of 128 tokens 7.1 ms, one CTA per SM 7.6); 8 only within
 // one CTA per SM (4096 x 2048, 128 tokens: eight 12.4 us, four 11.6; alone and with 32 tokens eight are 0.3 us faster, but the
-// 32-sequence step of Qwen3 is 2.70 ms with them, 2.63 with four).  Up to 32 tokens a share of less than 20 blocks of K is not
-// worth a second CTA on an SM (6144 gate/up pairs x 2048: two splits 14.7 us, unsplit 14.4; 6400 x 2560: 16.1, 16.7).
+// 32-sequence step of Qwen3 is 2.70 ms with them, 2.63 with four).  Up to 64 tokens a share of less than 20 blocks of K is not
+// worth it where most SMs would have two CTAs (6144 gate/up pairs x 2048, 96 tiles, 32 tokens: two splits 14.7 us, unsplit
+// 14.4; 16384 x 2048, 128 tiles, 64 tokens: 17.9, 17.6; but 10240 x 2048, 80 tiles: 14.0, 15.0; and 6400 x 2560: 16.1, 16.7).
 static int splits_two_per_sm(int tiles, int k, bool few) {
     const int sms = sm_count(), s = splits_for_tiles(tiles, k, 2 * sms, 4);
-    if (s == 2 && few && 2 * tiles > sms && k < 40 * TC_BK) return 1;
+    if (s == 2 && few && 8 * tiles > 5 * sms && k < 40 * TC_BK) return 1;
     return s == 4 ? std::max(s, splits_for_tiles(tiles, k, sms, 8)) : s;
 }
 int gemm_tc_splits(int n, int k) { return splits_two_per_sm((n + TC_BM - 1) / TC_BM, k, true); }
@@ -317,7 +318,7 @@ int gemm_tc_splits_for(int m, int n, int k, bool swiglu) {
         if (s == 4 && 4 * all <= room) return 4;
         return s >= 2 && 3 * all <= room ? 3 : std::min(s, 2);
     }
-    return splits_two_per_sm(tiles, k, m <= 32);
+    return splits_two_per_sm(tiles, k, m <= 64);
 }
 
 // Weights [rows][K], boxes of 64 elements x box_rows of each half (halves = 2: gate rows, then up rows).
